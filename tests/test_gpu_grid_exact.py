@@ -140,3 +140,28 @@ def test_generator_bit_exact(cuda, orc):
     api.generate_voltage(None, 7, 999, 2.5, _dev(torch, mu), 10, out, api.Dimensions(T, F, A, 1))
     assert np.array_equal(out.cpu().numpy().reshape(T, F, A),
                           orc.generate_voltage(7, 999, T, F, A, scale, mu, 10))
+
+
+@pytest.mark.parametrize("A,B,T,S", [(64, 8, 63, 64), (64, 9, 65, 1), (32, 40, 130, 7), (64, 63, 64, 10),
+                                     (64, 65, 129, 100), (128, 64, 70, 400), (256, 33, 66, 32), (64, 24, 400, 0),
+                                     (256, 1, 65, 0), (32, 128, 64, 0)])
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_tile_edges_bit_exact(cuda, orc, A, B, T, S, kernel):
+    """Beam counts around the lane columns (8) and the beam groups (64, 32 at
+    256 antennas), odd and even counts per lane, spectra around the tile (64)
+    and windows shorter and longer than it; S = 0 is the per-spectrum output."""
+    from beamform_project_b200 import api
+    torch = cuda
+    v = random_voltage(T, F, A, seed=T + B)
+    w = grid_weights(A, F, B, seed=B)
+    d = api.Dimensions(T, F, A, B)
+    dv, dw = _dev(torch, v), _dev(torch, w if kernel == 0 else tile_weights(w))
+    W = -(-T // S) if S else T
+    out = torch.full((W * F * B,), -1.0, dtype=torch.float32, device="cuda")
+    if S:
+        api.launch_packed_integrated_beamformer(kernel, None, dv, dw, out, d, S)
+        exp = orc.beamform_integrated(v, w, T, F, A, B, S)
+    else:
+        api.launch_packed_beamformer(kernel, None, dv, dw, out, d)
+        exp = orc.beamform(v, w, T, F, A, B)
+    assert np.array_equal(out.cpu().numpy().reshape(W, F, B), exp)
