@@ -25,11 +25,18 @@
 // precision.  Grid construction, clamping and interpolation are float32 with
 // the reference's operation order.
 //
-// Launches per window: (level kernel, select kernel) per level.  The level
-// kernel evaluates its points x channels (lane = point, warp = channel) and
-// writes one partial sum per (point, 64-channel group); the select kernel
-// (one CTA) adds the groups in order, takes the argmax and writes the next
-// level's points, or the window's direction and the next window's grid.
+// One launch per window and level.  A CTA takes 8 points and a group of 64
+// channels (lane = one of 8 points, one of 4 channels), writes one partial
+// sum per (point, group), and the CTA that finishes last adds the groups in
+// order, takes the argmax and writes the next level's points, or the
+// window's direction and the next window's grid.  What bounds it: the chain
+// of windows and levels, each a launch whose work (2e7 FP64 operations for a
+// 16 x 16 grid of 8 elements, 1 us of the FP64 pipe) is short, so the work is
+// spread thin (192 CTAs where 48 left two thirds of the SMs idle) and the
+// selection rides in the same launch and in all threads of its CTA.
+// Measured, 32 windows of 256 spectra, 64 antennas, 8 elements, 16 x 16 grid,
+// 2 refinements: 12.8 us per launch, 96 launches (21 us, and 27 us for a
+// selection kernel by one thread after each); the whole call 5.42 -> 1.92 ms.
 #include "bf_internal.cuh"
 #include "tracker_common.cuh"
 
@@ -53,7 +60,7 @@ struct SearchState {
     float cl, cm;          // running centre (l, m)
     float half_l, half_m;  // refinement half-pitch of the current level
     int n_points;          // points of the current level
-    int pad;
+    unsigned done;         // CTAs of the running level kernel that have written their sums
 };
 
 struct TrackParams {
@@ -76,25 +83,162 @@ __device__ __forceinline__ float2 clamp_disk(float l, float m) {
     return make_float2(l, m);
 }
 
+// The reference's 3-point interpolation (src/cpu_opt_beam_tracker.cpp:
+// 830-850): an offset only where denom > 0, clamped to [-0.5, 0.5].
+__device__ __forceinline__ float interp_offset(float pc, float p_up, float p_down) {
+    const float denom = __fadd_rn(__fsub_rn(p_down, __fmul_rn(2.0f, pc)), p_up);
+    if (!(denom > 0.0f)) return 0.0f;
+    const float d = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p_up, p_down)), denom);
+    return fminf(0.5f, fmaxf(-0.5f, d));
+}
+
+// Cell i of the G x G grid around (cl, cm).
+__device__ __forceinline__ float2 coarse_point(int i, float cl, float cm, int G, float fov_l, float fov_m) {
+    const float step_l = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_l), static_cast<float>(G - 1));
+    const float step_m = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_m), static_cast<float>(G - 1));
+    const float start_l = __fsub_rn(cl, fov_l), start_m = __fsub_rn(cm, fov_m);
+    const int u = i % G, v = i / G;
+    return clamp_disk(__fadd_rn(start_l, __fmul_rn(static_cast<float>(u), step_l)),
+                      __fadd_rn(start_m, __fmul_rn(static_cast<float>(v), step_m)));
+}
+
+constexpr int kLevelThreads = 256;
+constexpr int kPointTile = 8;        // points per CTA
+constexpr int kMaxDirect = 256;      // points whose powers fit the fixed shared array
+
+// What a level's selection needs beside the powers.
+struct SelectParams {
+    int n_groups, level, levels, G;
+    float fov_l, fov_m;
+    int interp;
+    float* dir_out;
+    int last_window;
+};
+
+// By every thread of the last CTA: the level's powers in float, as the
+// reference compares and interpolates them, their first maximum, and the next
+// level or window.  pw holds the powers (shared memory).
+__device__ __forceinline__ void select_level(const double* __restrict partial, float2* __restrict points,
+                                             SearchState* __restrict st, const SelectParams& q, int n,
+                                             float* __restrict pw) {
+    constexpr int kWarps = kLevelThreads / 32;
+    __shared__ float best_v[kWarps];
+    __shared__ int best_i[kWarps];
+    __shared__ float next[4];  // centre and half-pitches of the next level
+    const int tid = threadIdx.x, lane = tid & 31;
+    float bv = -INFINITY;
+    int bi = n;
+    for (int i = tid; i < n; i += kLevelThreads) {
+        double s = 0.0;
+        for (int g = 0; g < q.n_groups; ++g) s += __ldcg(partial + static_cast<size_t>(g) * kMaxPoints + i);
+        const float x = static_cast<float>(s);
+        pw[i] = x;
+        if (x > bv) { bv = x; bi = i; }  // first maximum: strict > over increasing index
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
+    }
+    if (lane == 0) {
+        best_v[tid >> 5] = bv;
+        best_i[tid >> 5] = bi;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < kWarps; ++w) {
+            if (best_v[w] > bv || (best_v[w] == bv && best_i[w] < bi)) { bv = best_v[w]; bi = best_i[w]; }
+        }
+        if (bi >= n) bi = 0;  // every power NaN-free and -inf: the first cell, as the reference
+        const float2 best = points[bi];
+        float cl = best.x, cm = best.y, half_l = st->half_l, half_m = st->half_m;
+        if (q.level == 0) {
+            if (q.levels == 0 && q.interp) {
+                const int u = bi % q.G, v = bi / q.G;
+                auto at = [&](int du, int dv) -> float {
+                    const int uu = u + du, vv = v + dv;
+                    return (uu < 0 || uu >= q.G || vv < 0 || vv >= q.G) ? 0.0f : pw[vv * q.G + uu];
+                };
+                const float pc = pw[bi];
+                const float du = interp_offset(pc, at(1, 0), at(-1, 0));
+                const float dv = interp_offset(pc, at(0, 1), at(0, -1));
+                const float step_l = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_l), static_cast<float>(q.G - 1));
+                const float step_m = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_m), static_cast<float>(q.G - 1));
+                const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, step_l)), __fadd_rn(cm, __fmul_rn(dv, step_m)));
+                cl = c.x;
+                cm = c.y;
+            }
+            half_l = __fdiv_rn(q.fov_l, static_cast<float>(q.G));
+            half_m = __fdiv_rn(q.fov_m, static_cast<float>(q.G));
+        } else if (q.interp) {
+            // the candidates' centre row and column, whichever candidate won
+            const float du = interp_offset(pw[4], pw[5], pw[3]);
+            const float dv = interp_offset(pw[4], pw[7], pw[1]);
+            const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, half_l)), __fadd_rn(cm, __fmul_rn(dv, half_m)));
+            cl = c.x;
+            cm = c.y;
+        }
+        if (q.level < q.levels) {
+            half_l = __fmul_rn(half_l, 0.5f);
+            half_m = __fmul_rn(half_m, 0.5f);
+        } else {
+            // the window's direction (direction_from_lm)
+            q.dir_out[0] = cl;
+            q.dir_out[1] = cm;
+            q.dir_out[2] = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(cl, cl), __fmul_rn(cm, cm))));
+        }
+        st->cl = cl;
+        st->cm = cm;
+        st->half_l = half_l;
+        st->half_m = half_m;
+        st->n_points = q.level < q.levels ? 9 : q.G * q.G;
+        st->done = 0;
+        next[0] = cl;
+        next[1] = cm;
+        next[2] = half_l;
+        next[3] = half_m;
+    }
+    __syncthreads();
+    if (q.level < q.levels) {
+        if (tid < 9) {
+            const float du = static_cast<float>(tid % 3 - 1), dv = static_cast<float>(tid / 3 - 1);
+            points[tid] = clamp_disk(__fadd_rn(next[0], __fmul_rn(du, next[2])),
+                                     __fadd_rn(next[1], __fmul_rn(dv, next[3])));
+        }
+    } else if (!q.last_window) {
+        for (int i = tid; i < q.G * q.G; i += kLevelThreads) {
+            points[i] = coarse_point(i, next[0], next[1], q.G, q.fov_l, q.fov_m);
+        }
+    }
+}
+
 // Bartlett or Capon power of window `b` at the points, summed over each
-// 64-channel group: partial[group][point].
+// 64-channel group (partial[group][point]: channels w, w + 8, ... of the
+// group first, then w = 0 .. 7), and the selection by the last CTA.
 template <int M>
-__global__ void __launch_bounds__(256) doa_level_kernel(TrackParams p, int b, const float2* __restrict points,
-                                                        const SearchState* __restrict state,
-                                                        double* __restrict partial) {
+__global__ void __launch_bounds__(kLevelThreads) doa_level_kernel(TrackParams p, int b, float2* __restrict points,
+                                                                  SearchState* __restrict state,
+                                                                  double* __restrict partial, SelectParams q) {
+    extern __shared__ float pw_large[];  // powers of grids above kMaxDirect points
+    __shared__ float pw_small[kMaxDirect];
+    __shared__ double red[kChanGroup][kPointTile];
+    __shared__ double red_w[8][kPointTile];
+    __shared__ int s_last;
     const int n_points = state->n_points;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pt = blockIdx.x * 32 + lane;
+    const int pl = lane & 7, cl = lane >> 3;
+    const int pt = blockIdx.x * kPointTile + pl;
     const int group = blockIdx.y;
-    __shared__ double red[8][32];
-    double acc = 0.0;
-    if (pt < n_points) {
-        const float2 lm = points[pt];
-        const double l = lm.x, m = lm.y;
-        // n as direction_from_lm forms it (float), for arrays with z != 0
-        const float nf = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(lm.x, lm.x), __fmul_rn(lm.y, lm.y))));
-        const double n = nf;
-        for (int f = group * kChanGroup + warp; f < min(p.n_freq, (group + 1) * kChanGroup); f += 8) {
+    const float2 lm = pt < n_points ? points[pt] : make_float2(0.f, 0.f);
+    const double l = lm.x, m = lm.y;
+    // n as direction_from_lm forms it (float), for arrays with z != 0
+    const double n = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(lm.x, lm.x), __fmul_rn(lm.y, lm.y))));
+#pragma unroll 1
+    for (int c = 4 * warp + cl; c < kChanGroup; c += 32) {
+        const int f = group * kChanGroup + c;
+        double pw = 0.0;
+        if (f < p.n_freq && pt < n_points) {
             const size_t cell = static_cast<size_t>(b) * p.n_freq + f;
             const double k = p.kw[f];
             Cd a[M];
@@ -113,158 +257,65 @@ __global__ void __launch_bounds__(256) doa_level_kernel(TrackParams p, int b, co
                 diag += X[r * M + r].re * mag[r];
                 double tr = 0.0, ti = 0.0;
 #pragma unroll
-                for (int c = r + 1; c < M; ++c) {
-                    const Cd x = X[r * M + c];
-                    tr += x.re * a[c].re - x.im * a[c].im;
-                    ti += x.re * a[c].im + x.im * a[c].re;
+                for (int e = r + 1; e < M; ++e) {
+                    const Cd x = X[r * M + e];
+                    tr += x.re * a[e].re - x.im * a[e].im;
+                    ti += x.re * a[e].im + x.im * a[e].re;
                 }
                 off += a[r].re * tr + a[r].im * ti;  // Re(conj(a_r) * (X a)_r upper part)
             }
-            double pw = diag + 2.0 * off;
+            pw = diag + 2.0 * off;
             if (p.capon) pw = (p.ok[cell] && pw > 0.0) ? 1.0 / pw : 0.0;
             if (!isfinite(pw)) pw = 0.0;
-            acc += pw;
         }
+        red[c][pl] = pw;
     }
-    red[warp][lane] = acc;
     __syncthreads();
-    if (warp == 0 && pt < n_points) {
+    if (threadIdx.x < 8 * kPointTile) {
+        const int w = threadIdx.x >> 3;
+        double acc = 0.0;
+#pragma unroll
+        for (int i = 0; i < kChanGroup / 8; ++i) acc += red[w + 8 * i][threadIdx.x & 7];
+        red_w[w][threadIdx.x & 7] = acc;
+    }
+    __syncthreads();
+    if (threadIdx.x < kPointTile && blockIdx.x * kPointTile + threadIdx.x < n_points) {
         double s = 0.0;
-        for (int w = 0; w < 8; ++w) s += red[w][lane];
-        partial[static_cast<size_t>(group) * kMaxPoints + pt] = s;
-    }
-}
-
-// The reference's 3-point interpolation (src/cpu_opt_beam_tracker.cpp:
-// 830-850): an offset only where denom > 0, clamped to [-0.5, 0.5].
-__device__ __forceinline__ float interp_offset(float pc, float p_up, float p_down) {
-    const float denom = __fadd_rn(__fsub_rn(p_down, __fmul_rn(2.0f, pc)), p_up);
-    if (!(denom > 0.0f)) return 0.0f;
-    const float d = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p_up, p_down)), denom);
-    return fminf(0.5f, fmaxf(-0.5f, d));
-}
-
-__device__ __forceinline__ void coarse_grid(SearchState* st, float2* points, float cl, float cm, int G, float fov_l,
-                                            float fov_m) {
-    const float step_l = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_l), static_cast<float>(G - 1));
-    const float step_m = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_m), static_cast<float>(G - 1));
-    const float start_l = __fsub_rn(cl, fov_l), start_m = __fsub_rn(cm, fov_m);
-    for (int i = 0; i < G * G; ++i) {
-        const int u = i % G, v = i / G;
-        points[i] = clamp_disk(__fadd_rn(start_l, __fmul_rn(static_cast<float>(u), step_l)),
-                               __fadd_rn(start_m, __fmul_rn(static_cast<float>(v), step_m)));
-    }
-    st->n_points = G * G;
-}
-
-__device__ __forceinline__ void refine_grid(SearchState* st, float2* points) {
-    for (int dv = -1; dv <= 1; ++dv) {
-        for (int du = -1; du <= 1; ++du) {
-            points[(dv + 1) * 3 + (du + 1)] =
-                clamp_disk(__fadd_rn(st->cl, __fmul_rn(static_cast<float>(du), st->half_l)),
-                           __fadd_rn(st->cm, __fmul_rn(static_cast<float>(dv), st->half_m)));
-        }
-    }
-    st->n_points = 9;
-}
-
-// One CTA: the level's powers, argmax and the next level or window.
-__global__ void __launch_bounds__(256) doa_select_kernel(const double* __restrict partial, int n_groups,
-                                                         float2* __restrict points, SearchState* __restrict st,
-                                                         int level, int levels, int G, float fov_l, float fov_m,
-                                                         int interp, float* __restrict dir_out, int last_window) {
-    __shared__ float pw[kMaxPoints];
-    __shared__ float best_v[256];
-    __shared__ int best_i[256];
-    const int n = st->n_points;
-    // powers in float, as the reference compares and interpolates them
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        double s = 0.0;
-        for (int g = 0; g < n_groups; ++g) s += partial[static_cast<size_t>(g) * kMaxPoints + i];
-        pw[i] = static_cast<float>(s);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red_w[w][threadIdx.x];
+        partial[static_cast<size_t>(group) * kMaxPoints + blockIdx.x * kPointTile + threadIdx.x] = s;
+        __threadfence();
     }
     __syncthreads();
-    // first maximum: strict > over increasing index
-    float bv = -INFINITY;
-    int bi = n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        if (pw[i] > bv) { bv = pw[i]; bi = i; }
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&state->done, 1u) + 1 == gridDim.x * gridDim.y;
+        __threadfence();
     }
-    best_v[threadIdx.x] = bv;
-    best_i[threadIdx.x] = bi;
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int t = 1; t < blockDim.x; ++t) {
-        if (best_v[t] > bv || (best_v[t] == bv && best_i[t] < bi)) { bv = best_v[t]; bi = best_i[t]; }
-    }
-    if (bi >= n) bi = 0;  // every power NaN-free and -inf: the first cell, as the reference
-    const float2 best = points[bi];
-    float cl = best.x, cm = best.y;
-    if (level == 0) {
-        if (levels == 0 && interp) {
-            const int u = bi % G, v = bi / G;
-            auto at = [&](int du, int dv) -> float {
-                const int uu = u + du, vv = v + dv;
-                return (uu < 0 || uu >= G || vv < 0 || vv >= G) ? 0.0f : pw[vv * G + uu];
-            };
-            const float pc = pw[bi];
-            const float du = interp_offset(pc, at(1, 0), at(-1, 0));
-            const float dv = interp_offset(pc, at(0, 1), at(0, -1));
-            const float step_l = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_l), static_cast<float>(G - 1));
-            const float step_m = G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, fov_m), static_cast<float>(G - 1));
-            const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, step_l)), __fadd_rn(cm, __fmul_rn(dv, step_m)));
-            cl = c.x;
-            cm = c.y;
-        }
-        st->half_l = __fdiv_rn(fov_l, static_cast<float>(G));
-        st->half_m = __fdiv_rn(fov_m, static_cast<float>(G));
-    } else {
-        if (interp) {
-            // the candidates' centre row and column, whichever candidate won
-            const float du = interp_offset(pw[4], pw[5], pw[3]);
-            const float dv = interp_offset(pw[4], pw[7], pw[1]);
-            const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, st->half_l)),
-                                        __fadd_rn(cm, __fmul_rn(dv, st->half_m)));
-            cl = c.x;
-            cm = c.y;
-        }
-    }
-    st->cl = cl;
-    st->cm = cm;
-    if (level < levels) {
-        st->half_l = __fmul_rn(st->half_l, 0.5f);
-        st->half_m = __fmul_rn(st->half_m, 0.5f);
-        refine_grid(st, points);
-        return;
-    }
-    // the window's direction (direction_from_lm) and the next window's grid
-    dir_out[0] = cl;
-    dir_out[1] = cm;
-    dir_out[2] = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(cl, cl), __fmul_rn(cm, cm))));
-    if (!last_window) coarse_grid(st, points, cl, cm, G, fov_l, fov_m);
+    if (s_last) select_level(partial, points, state, q, n_points, n_points <= kMaxDirect ? pw_small : pw_large);
 }
 
 __global__ void doa_track_init_kernel(SearchState* st, float2* points, float l0, float m0, int G, float fov_l,
                                       float fov_m) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) coarse_grid(st, points, l0, m0, G, fov_l, fov_m);
+    for (int i = threadIdx.x; i < G * G; i += blockDim.x) points[i] = coarse_point(i, l0, m0, G, fov_l, fov_m);
+    if (threadIdx.x == 0) {
+        st->n_points = G * G;
+        st->done = 0;
+    }
 }
 
 template <int M>
-bf_status launch_level(cudaStream_t stream, const TrackParams& p, int b, const float2* points, const SearchState* st,
-                       double* partial, int n_points_max, int n_groups) {
-    const dim3 grid(static_cast<unsigned>((n_points_max + 31) / 32), static_cast<unsigned>(n_groups));
-    doa_level_kernel<M><<<grid, 256, 0, stream>>>(p, b, points, st, partial);
-    return cuda_status(cudaGetLastError(), "doa_level_kernel launch");
-}
-
-template <int M>
-bf_status dispatch_level(int m, cudaStream_t stream, const TrackParams& p, int b, const float2* points,
-                         const SearchState* st, double* partial, int n_points_max, int n_groups) {
+bf_status launch_level(int m, cudaStream_t stream, const TrackParams& p, int b, float2* points, SearchState* st,
+                       double* partial, int n_points, const SelectParams& q) {
     if constexpr (M > kMaxM) {
         return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 16 elements after smoothing");
     } else {
-        if (m == M) return launch_level<M>(stream, p, b, points, st, partial, n_points_max, n_groups);
-        return dispatch_level<M + 1>(m, stream, p, b, points, st, partial, n_points_max, n_groups);
+        if (m != M) return launch_level<M + 1>(m, stream, p, b, points, st, partial, n_points, q);
+        const dim3 grid(static_cast<unsigned>((n_points + kPointTile - 1) / kPointTile),
+                        static_cast<unsigned>(q.n_groups));
+        const size_t smem = n_points > kMaxDirect ? n_points * sizeof(float) : 0;
+        doa_level_kernel<M><<<grid, kLevelThreads, smem, stream>>>(p, b, points, st, partial, q);
+        return cuda_status(cudaGetLastError(), "doa_level_kernel launch");
     }
 }
 
@@ -313,15 +364,20 @@ bf_status launch_doa_track(cudaStream_t stream, const uint8_t* v, const float* p
     p.M = M;
     p.capon = c.estimator != 0;
     const int G = static_cast<int>(c.grid), L = static_cast<int>(c.levels);
-    doa_track_init_kernel<<<1, 32, 0, stream>>>(st, points, c.prior_l, c.prior_m, G, c.fov_l, c.fov_m);
+    doa_track_init_kernel<<<1, 256, 0, stream>>>(st, points, c.prior_l, c.prior_m, G, c.fov_l, c.fov_m);
     BF_RETURN_IF(cuda_status(cudaGetLastError(), "doa_track_init_kernel launch"));
+    SelectParams q{};
+    q.n_groups = static_cast<int>(groups);
+    q.levels = L;
+    q.G = G;
+    q.fov_l = c.fov_l;
+    q.fov_m = c.fov_m;
+    q.interp = c.interp != 0;
     for (int b = 0; b < B; ++b) {
-        for (int level = 0; level <= L; ++level) {
-            const int n_max = level == 0 ? G * G : 9;
-            BF_RETURN_IF(dispatch_level<1>(M, stream, p, b, points, st, partial, n_max, static_cast<int>(groups)));
-            doa_select_kernel<<<1, 256, 0, stream>>>(partial, static_cast<int>(groups), points, st, level, L, G,
-                                                     c.fov_l, c.fov_m, c.interp != 0, dirs + 3 * b, b + 1 == B);
-            BF_RETURN_IF(cuda_status(cudaGetLastError(), "doa_select_kernel launch"));
+        q.dir_out = dirs + 3 * b;
+        q.last_window = b + 1 == B;
+        for (q.level = 0; q.level <= L; ++q.level) {
+            BF_RETURN_IF(launch_level<1>(M, stream, p, b, points, st, partial, q.level == 0 ? G * G : 9, q));
         }
     }
     if (intensity == nullptr) return BF_OK;

@@ -267,3 +267,50 @@ def test_adaptive_tracker_follows_reference_search(cuda, ref, orc, A, capon, sub
     same = np.all(got == ref_dirs, axis=1)
     for w in np.nonzero(same)[0]:
         assert np.array_equal(got_I[w * K:(w + 1) * K], ref_I[w * K:(w + 1) * K])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("G,M,capon", [(9, 8, False), (24, 12, False), (24, 5, True), (3, 16, True)])
+def test_adaptive_tracker_takes_the_grid_maximum(cuda, orc, G, M, capon):
+    """Without refinement or interpolation each window's direction is the
+    cell of largest power: grids around the point tile (8 points per CTA) and
+    above the fixed shared array (256 points), against FP64 powers.  The
+    search adds FP64 powers of FP32 steering components and compares them as
+    float32 (2^-24 relative), so any cell within 1e-6 of the maximum is right."""
+    from beamform_project_b200 import api
+    torch = cuda
+    A, K, W, fov, load, lam = 64, 128, 3, 0.2, 1e-3, 0.9
+    pos, freq, kw = geometry(A)
+    v = source_voltage(K * W, A, [(0.07, 3.0, 0.0)], seed=G + M)
+    d = api.Dimensions(K * W, F, A, 1)
+    cfg = api.doa_track_config(K, subarray=M, capon=capon, grid=G, levels=0, interp=False, fov_l=fov, fov_m=fov,
+                               forgetting=lam, diag_load=load)
+    ws = torch.empty(api.doa_track_workspace_bytes(d, cfg), dtype=torch.uint8, device="cuda")
+    dirs = torch.zeros(W * 3, dtype=torch.float32, device="cuda")
+    api.doa_track(None, torch.from_numpy(v).cuda(), torch.from_numpy(pos).cuda(), torch.from_numpy(kw).cuda(), d, cfg,
+                  dirs, None, ws)
+    got = dirs.cpu().numpy().reshape(W, 3)
+    R = orc.covariance_blocks(v, K).astype(np.float64)
+    R = (R[..., 0] + 1j * R[..., 1]) / K
+    L = A - M + 1
+    S = sum(R[:, :, i:i + M, i:i + M] for i in range(L)) / L
+    if L > 1:
+        S = (S + S[:, :, ::-1, ::-1].conj()) / 2
+    eps = load * np.trace(S, axis1=2, axis2=3).real / M
+    for w in range(1, W):
+        S[w] = lam * S[w - 1] + (1 - lam) * S[w]
+        eps[w] = lam * eps[w - 1] + (1 - lam) * eps[w]
+    X = np.linalg.inv(S + eps[..., None, None] * np.eye(M)) if capon else S
+    centre = np.zeros(2, np.float32)
+    for w in range(W):
+        step = np.float32(2 * np.float32(fov)) / np.float32(G - 1)
+        ax = np.arange(G).astype(np.float32) * step
+        lm = np.stack(np.meshgrid(centre[0] - np.float32(fov) + ax, centre[1] - np.float32(fov) + ax), -1).reshape(-1, 2)
+        ph = -kw[:, None, None] * (lm.astype(np.float64) @ pos[:M, :2].astype(np.float64).T)[None]
+        a = np.exp(1j * ph)
+        p = np.einsum("fnr,frc,fnc->fn", a.conj(), X[w], a, optimize=True).real
+        p = (1.0 / p if capon else p).sum(0)
+        cell = np.argmin(np.abs(lm - got[w, :2]).sum(1))
+        assert np.array_equal(lm[cell], got[w, :2])
+        assert p[cell] >= p.max() * (1 - 1e-6)
+        centre = got[w, :2]
