@@ -25,13 +25,31 @@
 //     bytes of two rows; the K order of the contraction is permuted to match
 //     the decode (only the weights need to follow it).
 // A CTA of 8 warps takes 8 consecutive channels (512 contiguous bytes per
-// spectrum at 64 antennas) for one window; per-spectrum powers are staged in
-// shared memory so each spectrum's 8 channels are written as one 32-byte
-// sector.
+// spectrum at 64 antennas), a warp one channel, in blocks of 16 spectra.  The
+// FP64 delays of the CTA's windows are formed once and each weight once per
+// warp (a lane forms the two antennas of a fragment word), passed to the
+// fragment columns through shared memory: forming them per fragment repeated
+// each weight four times in half of the lanes.  Two forms:
+//   * long windows, one per CTA: two blocks' rows in registers, the next two
+//     on their way;
+//   * short windows, a run of up to 16 per CTA: each lane fills a ring of
+//     kDepth blocks for itself with cp.async and reads it back itself, so the
+//     loads run ahead over the window ends without registers or barriers.
+// Per-spectrum powers are staged four blocks at a time so that each
+// spectrum's 8 channels are written as one 32-byte sector.
+// What bounds it: instruction issue with HBM close behind for long windows;
+// for windows of 10 spectra the weights' arithmetic and the six empty rows of
+// each block.
+// Measured at 64 antennas: 15360 spectra in windows of 10 with both outputs
+// 0.252 ms (0.819 ms with weights formed per fragment and one window per
+// CTA), 32000 in windows of 320 0.166 ms (0.190), 131072 in windows of 1024
+// 0.637 ms = 4.4 TB/s (0.666).
 #include "bf_internal.cuh"
 #include "tracker_common.cuh"
 
 #include <cuda_fp16.h>
+
+#include <algorithm>
 
 namespace bf {
 namespace {
@@ -39,81 +57,191 @@ namespace {
 using namespace trk;
 
 constexpr int kChannelsPerCta = 8;
+constexpr int kMaxRun = 16;         // windows per CTA
+constexpr int kRunSpectra = 160;    // a run is as many windows as fit, one at least
+constexpr int kWantedCtas = 4 * 4 * 148;
+// Longest window of the ring form: windows of 100 take 75 us in it and 77 us
+// in the long form (9999 spectra), windows of 320 179 and 166 us (32000).
+constexpr int kShortWindow = 64;
+constexpr int kStageBlocks = 4;     // blocks of per-spectrum powers between barriers
 
+// Blocks of 16 spectra in a warp's ring (1 KB each at 64 antennas).
 template <int A>
+__host__ __device__ constexpr int ring_depth() { return A == 32 ? 8 : A == 64 ? 4 : A == 128 ? 3 : 2; }
+
+template <int N>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool on) {
+    // a source size of 0 reads nothing and zero-fills
+    if constexpr (N == 8) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(on ? 8 : 0) : "memory");
+    } else {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0)
+                     : "memory");
+    }
+}
+
+// Blocks of a run of windows in order: 16 spectra at a time, a window's last
+// block as short as the window leaves it.
+struct BlockCursor {
+    int win, t, end;  // window, first spectrum of the block, end of the window
+    __device__ __forceinline__ void start(int w, int spectra, int n_time) {
+        win = w;
+        t = w * spectra;
+        end = min(t + spectra, n_time);
+    }
+    __device__ __forceinline__ void next(int spectra, int n_time) {
+        t += 16;
+        if (t >= end) start(win + 1, spectra, n_time);
+    }
+};
+
+template <int A, bool kRuns>
 __global__ void __launch_bounds__(kChannelsPerCta * 32)
 tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ pos,
                       const double* __restrict__ kw, const float* __restrict__ dirs,
                       float* __restrict__ intensity, float* __restrict__ integrated, int n_time,
-                      int n_freq, int spectra) {
+                      int n_freq, int spectra, int n_windows, int run) {
     constexpr int NW = A / 16;          // 32-bit words per thread per spectrum
     constexpr int kBytes = A / 4;       // bytes per thread per spectrum
-    __shared__ float stage[16][kChannelsPerCta];
+    constexpr int kDepth = ring_depth<A>();
+    constexpr int kCopy = A == 32 ? 8 : 16, kCopies = kBytes / kCopy;
+    constexpr int kSlot = 16 * A;       // bytes of a block: [row half][copy][lane]
+    extern __shared__ uint4 smem_raw[];
+    uint8_t* ring_all = reinterpret_cast<uint8_t*>(smem_raw);               // [8 warps][kDepth][kSlot] (kRuns)
+    uint32_t* parts_all = reinterpret_cast<uint32_t*>(ring_all + (kRuns ? 8 * kDepth * kSlot : 0));  // [8][4][A / 2]
+    double* delays = reinterpret_cast<double*>(parts_all + 8 * 2 * A);      // [run][A]
+    float* stage = reinterpret_cast<float*>(delays + run * A);              // [2][kStageBlocks][16][8], with intensity
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
-    const int win = blockIdx.x;
+    const int w_begin = blockIdx.x * run, w_end = min(w_begin + run, n_windows);
     const int f = blockIdx.y * kChannelsPerCta + warp;
     const bool fvalid = f < n_freq;
 
-    // B fragments for this window: column g in (re_hi, im_hi, re_lo, im_lo, 0...).
-    uint32_t bfrag[NW][2][2];
-    {
-        const bool used = g < 4 && fvalid;
-        const bool is_im = (g & 1) != 0, is_lo = (g >> 1) != 0;
-        const double k = fvalid ? kw[f] : 0.0;
-        const double dx = dirs[3 * win], dy = dirs[3 * win + 1], dz = dirs[3 * win + 2];
+    // rows g and g + 8 of the block at t, zero past the window's end
+    const size_t row_bytes = static_cast<size_t>(n_freq) * A;
+    const uint8_t* lane_src = v + static_cast<size_t>(fvalid ? f : 0) * A + q * kBytes;
+    auto load_rows = [&](int t, int end, uint32_t (&wd)[2][NW]) {
 #pragma unroll
-        for (int j = 0; j < NW; ++j) {
+        for (int h = 0; h < 2; ++h) {
+            const bool on = fvalid && t + g + 8 * h < end;
+            const uint8_t* src = lane_src + static_cast<size_t>(t + g + 8 * h) * row_bytes;
+            if constexpr (A == 32) {
+                const uint2 x = on ? __ldg(reinterpret_cast<const uint2*>(src)) : make_uint2(0, 0);
+                wd[h][0] = x.x; wd[h][1] = x.y;
+            } else {
 #pragma unroll
-            for (int s = 0; s < 2; ++s) {
-                const int a0 = q * kBytes + 4 * j + s, a1 = a0 + 2;
-                uint32_t xr = 0, xi = 0;
-                if (used) {
-                    const float2 w0 = steering_weight(pos, a0, k, dx, dy, dz);
-                    const float2 w1 = steering_weight(pos, a1, k, dx, dy, dz);
-                    // re: xr*wr - xi*wi ; im: xr*wi + xi*wr
-                    const float cr0 = is_im ? w0.y : w0.x, cr1 = is_im ? w1.y : w1.x;
-                    const float ci0 = is_im ? w0.x : -w0.y, ci1 = is_im ? w1.x : -w1.y;
-                    xr = split_part(cr0, is_lo) | (static_cast<uint32_t>(split_part(cr1, is_lo)) << 16);
-                    xi = split_part(ci0, is_lo) | (static_cast<uint32_t>(split_part(ci1, is_lo)) << 16);
+                for (int c = 0; c < kCopies; ++c) {
+                    const uint4 x = on ? __ldg(reinterpret_cast<const uint4*>(src) + c) : make_uint4(0, 0, 0, 0);
+                    wd[h][4 * c] = x.x; wd[h][4 * c + 1] = x.y; wd[h][4 * c + 2] = x.z; wd[h][4 * c + 3] = x.w;
                 }
-                bfrag[j][s][0] = xr;
-                bfrag[j][s][1] = xi;
-            }
-        }
-    }
-
-    const int t_begin = win * spectra;
-    const int t_end = min(t_begin + spectra, n_time);
-    float acc = 0.f;
-    // Rows g and g+8 of the 16-spectrum block starting at tb (zero past the window).
-    auto load_rows = [&](int tb, uint32_t (&wg)[NW], uint32_t (&wg8)[NW]) {
-        const int tg = tb + g, tg8 = tb + g + 8;
-        const uint8_t* rg = v + (static_cast<size_t>(tg) * n_freq + f) * A + q * kBytes;
-        const uint8_t* rg8 = v + (static_cast<size_t>(tg8) * n_freq + f) * A + q * kBytes;
-        const bool vg = fvalid && tg < t_end, vg8 = fvalid && tg8 < t_end;
-        if constexpr (A == 32) {
-            const uint2 x0 = vg ? __ldg(reinterpret_cast<const uint2*>(rg)) : make_uint2(0, 0);
-            const uint2 x1 = vg8 ? __ldg(reinterpret_cast<const uint2*>(rg8)) : make_uint2(0, 0);
-            wg[0] = x0.x; wg[1] = x0.y; wg8[0] = x1.x; wg8[1] = x1.y;
-        } else {
-#pragma unroll
-            for (int c = 0; c < NW / 4; ++c) {
-                const uint4 x0 = vg ? __ldg(reinterpret_cast<const uint4*>(rg) + c) : make_uint4(0, 0, 0, 0);
-                const uint4 x1 = vg8 ? __ldg(reinterpret_cast<const uint4*>(rg8) + c) : make_uint4(0, 0, 0, 0);
-                wg[4 * c] = x0.x; wg[4 * c + 1] = x0.y; wg[4 * c + 2] = x0.z; wg[4 * c + 3] = x0.w;
-                wg8[4 * c] = x1.x; wg8[4 * c + 1] = x1.y; wg8[4 * c + 2] = x1.z; wg8[4 * c + 3] = x1.w;
             }
         }
     };
-    auto process = [&](const uint32_t (&wg)[NW], const uint32_t (&wg8)[NW], int tb) {
+    // the ring: loads of the run's blocks in order, kDepth - 1 ahead
+    uint8_t* ring = ring_all + warp * kDepth * kSlot;
+    const uint32_t ring_at = static_cast<uint32_t>(__cvta_generic_to_shared(ring)) + lane * kCopy;
+    BlockCursor ahead;
+    int ahead_slot = 0;
+    auto ring_load = [&]() {
+        if (ahead.win < w_end) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int t = ahead.t + g + 8 * h;
+                const bool on = fvalid && t < ahead.end;
+                const uint8_t* src = lane_src + (on ? t : ahead.t) * row_bytes;
+#pragma unroll
+                for (int c = 0; c < kCopies; ++c) {
+                    copy_async<kCopy>(ring_at + ahead_slot * kSlot + (h * kCopies + c) * 32 * kCopy, src + c * kCopy, on);
+                }
+            }
+            ahead.next(spectra, n_time);
+        }
+        if (++ahead_slot == kDepth) ahead_slot = 0;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto ring_read = [&](int slot, uint32_t (&wd)[2][NW]) {
+        const uint8_t* src = ring + slot * kSlot + lane * kCopy;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if constexpr (A == 32) {
+                const uint2 x = *reinterpret_cast<const uint2*>(src + h * 32 * kCopy);
+                wd[h][0] = x.x; wd[h][1] = x.y;
+            } else {
+#pragma unroll
+                for (int c = 0; c < kCopies; ++c) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(src + (h * kCopies + c) * 32 * kCopy);
+                    wd[h][4 * c] = x.x; wd[h][4 * c + 1] = x.y; wd[h][4 * c + 2] = x.z; wd[h][4 * c + 3] = x.w;
+                }
+            }
+        }
+    };
+
+    BlockCursor cur;
+    cur.start(w_begin, spectra, n_time);
+    uint32_t wa[2][NW], wb[2][NW];
+    if constexpr (kRuns) {
+        ahead = cur;
+#pragma unroll
+        for (int i = 0; i < kDepth - 1; ++i) ring_load();
+    } else {
+        load_rows(cur.t, cur.end, wa);
+        load_rows(cur.t + 16, cur.end, wb);
+    }
+    for (int i = threadIdx.x; i < (w_end - w_begin) * A; i += kChannelsPerCta * 32) {
+        const float* d = dirs + 3 * (w_begin + i / A);
+        delays[i] = steering_delay(pos, i % A, d[0], d[1], d[2]);
+    }
+    __syncthreads();
+
+    // B fragments of a window: column g in (re_hi, im_hi, re_lo, im_lo, 0...).
+    const double k = fvalid ? kw[f] : 0.0;
+    uint32_t* parts = parts_all + warp * 2 * A;  // rows re_hi, im_hi, re_lo, im_lo of words (a, a + 2)
+    uint32_t bfrag[NW][2][2];
+    auto form_weights = [&](int w) {
+        __syncwarp();  // the previous window's words are read
+        const double* dl = delays + (w - w_begin) * A;
+#pragma unroll
+        for (int i = 0; i < (A / 2 + 31) / 32; ++i) {
+            const int word = lane + 32 * i, a0 = 4 * (word >> 1) + (word & 1);
+            if (word < A / 2) {
+                const float2 w0 = steering_from_delay(k, dl[a0]), w1 = steering_from_delay(k, dl[a0 + 2]);
+#pragma unroll
+                for (int lo = 0; lo < 2; ++lo) {
+                    parts[lo * A + word] = split_part(w0.x, lo) | (static_cast<uint32_t>(split_part(w1.x, lo)) << 16);
+                    parts[lo * A + A / 2 + word] =
+                        split_part(w0.y, lo) | (static_cast<uint32_t>(split_part(w1.y, lo)) << 16);
+                }
+            }
+        }
+        __syncwarp();
+        // re: xr * wr - xi * wi; im: xr * wi + xi * wr (column g < 4; the rest are zero)
+        const bool is_im = (g & 1) != 0;
+        const uint32_t flip = is_im ? 0u : 0x80008000u;
+        const uint32_t* row_r = parts + ((g >> 1) & 1) * A + (is_im ? A / 2 : 0) + q * 2 * NW;
+        const uint32_t* row_i = parts + ((g >> 1) & 1) * A + (is_im ? 0 : A / 2) + q * 2 * NW;
+#pragma unroll
+        for (int j = 0; j < NW; j += 2) {
+            const uint4 r4 = *reinterpret_cast<const uint4*>(row_r + 2 * j);
+            const uint4 i4 = *reinterpret_cast<const uint4*>(row_i + 2 * j);
+            const uint32_t wr[4] = {r4.x, r4.y, r4.z, r4.w}, wi[4] = {i4.x, i4.y, i4.z, i4.w};
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                bfrag[j + (s >> 1)][s & 1][0] = g < 4 ? wr[s] : 0u;
+                bfrag[j + (s >> 1)][s & 1][1] = g < 4 ? wi[s] ^ flip : 0u;
+            }
+        }
+    };
+
+    float acc = 0.f;
+    // One block: its spectra's powers into the window sum and the stage.
+    auto process = [&](const uint32_t (&wd)[2][NW], int staged) {
         float d[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
         for (int j = 0; j < NW; ++j) {
             uint32_t re02g, im02g, re13g, im13g, re02h, im02h, re13h, im13h;
-            decode_word(wg[j], re02g, im02g, re13g, im13g);
-            decode_word(wg8[j], re02h, im02h, re13h, im13h);
+            decode_word(wd[0][j], re02g, im02g, re13g, im13g);
+            decode_word(wd[1][j], re02h, im02h, re13h, im13h);
             mma_16816(d, re02g, re02h, im02g, im02h, bfrag[j][0][0], bfrag[j][0][1]);
             mma_16816(d, re13g, re13h, im13g, im13h, bfrag[j][1][0], bfrag[j][1][1]);
         }
@@ -125,48 +253,108 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
         const float re_h = d[2] + p[2], im_h = d[3] + p[3];
         const float pow_g = re_g * re_g + im_g * im_g;
         const float pow_h = re_h * re_h + im_h * im_h;
-        if (q == 0) acc += pow_g + pow_h;
-        if (intensity != nullptr) {
-            if (q == 0) {
-                stage[g][warp] = pow_g;
-                stage[g + 8][warp] = pow_h;
+        if (q == 0) {
+            acc += pow_g + pow_h;
+            if (intensity != nullptr) {
+                float* st = stage + staged * 16 * kChannelsPerCta + warp;
+                st[g * kChannelsPerCta] = pow_g;
+                st[(g + 8) * kChannelsPerCta] = pow_h;
             }
-            __syncthreads();
-            if (threadIdx.x < 16 * kChannelsPerCta) {
-                const int r = threadIdx.x / kChannelsPerCta, c = threadIdx.x % kChannelsPerCta;
-                const int fo = blockIdx.y * kChannelsPerCta + c;
-                if (tb + r < t_end && fo < n_freq) {
-                    intensity[static_cast<size_t>(tb + r) * n_freq + fo] = stage[r][c];
-                }
-            }
-            __syncthreads();
         }
     };
-    // software pipeline: the next two blocks' loads are in flight while two
-    // blocks compute (blocks are still summed one by one in increasing time)
-    uint32_t wa[NW], wa8[NW], wb[NW], wb8[NW];
-    load_rows(t_begin, wa, wa8);
-    load_rows(t_begin + 16, wb, wb8);
-    for (int tb = t_begin; tb < t_end; tb += 32) {
-        uint32_t na[NW], na8[NW], nb[NW], nb8[NW];
-        load_rows(tb + 32, na, na8);
-        load_rows(tb + 48, nb, nb8);
-        process(wa, wa8, tb);
-        if (tb + 16 < t_end) process(wb, wb8, tb + 16);  // uniform across the CTA
-#pragma unroll
-        for (int j = 0; j < NW; ++j) {
-            wa[j] = na[j];
-            wa8[j] = na8[j];
-            wb[j] = nb[j];
-            wb8[j] = nb8[j];
+    auto finish_window = [&](int w) {
+        if (integrated == nullptr) return;
+        float sum = acc;
+        sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        if (lane == 0 && fvalid) integrated[static_cast<size_t>(w) * n_freq + f] = sum;
+    };
+    // Writes out kStageBlocks staged blocks from `first` on.  One barrier per
+    // call: a buffer is written again only after the barrier of the other
+    // one, which every thread reaches after its reads here.
+    auto write_staged = [&](BlockCursor first, int buf) {
+        __syncthreads();
+        const int c = threadIdx.x % kChannelsPerCta, fo = blockIdx.y * kChannelsPerCta + c;
+        const int r = threadIdx.x / kChannelsPerCta;
+        for (int b = 0; b < kStageBlocks && first.win < w_end; ++b) {
+            if (r < 16 && first.t + r < first.end && fo < n_freq) {
+                intensity[static_cast<size_t>(first.t + r) * n_freq + fo] =
+                    stage[((buf * kStageBlocks + b) * 16 + r) * kChannelsPerCta + c];
+            }
+            first.next(spectra, n_time);
         }
+    };
+
+    if constexpr (kRuns) {
+        int slot = 0;
+        for (int buf = 0; cur.win < w_end; buf ^= 1) {
+            const BlockCursor first = cur;
+#pragma unroll 1
+            for (int b = 0; b < kStageBlocks && cur.win < w_end; ++b) {
+                ring_load();
+                asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+                if (cur.t == cur.win * spectra) {
+                    form_weights(cur.win);
+                    acc = 0.f;
+                }
+                ring_read(slot, wa);
+                if (++slot == kDepth) slot = 0;
+                process(wa, buf * kStageBlocks + b);
+                if (cur.t + 16 >= cur.end) finish_window(cur.win);
+                cur.next(spectra, n_time);
+            }
+            if (intensity != nullptr) write_staged(first, buf);
+        }
+    } else {
+        // the next two blocks' loads are in flight while two blocks compute
+        // (blocks are still summed one by one in increasing time)
+        form_weights(w_begin);
+        BlockCursor first = cur;
+        int staged = 0;
+        for (; cur.t < cur.end; cur.t += 32) {
+            uint32_t na[2][NW], nb[2][NW];
+            load_rows(cur.t + 32, cur.end, na);
+            load_rows(cur.t + 48, cur.end, nb);
+            process(wa, staged);
+            if (cur.t + 16 < cur.end) process(wb, staged + 1);  // uniform across the CTA
+            if (intensity != nullptr) {
+                staged = (staged + 2) % (2 * kStageBlocks);
+                if (staged % kStageBlocks == 0 || cur.t + 32 >= cur.end) {
+                    write_staged(first, (staged - 1 + 2 * kStageBlocks) % (2 * kStageBlocks) / kStageBlocks);
+                    first.t = cur.t + 32;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                for (int j = 0; j < NW; ++j) {
+                    wa[h][j] = na[h][j];
+                    wb[h][j] = nb[h][j];
+                }
+            }
+        }
+        finish_window(w_begin);
     }
-    if (integrated != nullptr) {
-        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-        if (lane == 0 && fvalid) integrated[static_cast<size_t>(win) * n_freq + f] = acc;
-    }
+}
+
+template <int A>
+bf_status launch_stream(cudaStream_t stream, const uint8_t* v, const float* pos, const double* k, const float* dirs,
+                        float* intensity, float* integrated, int T, int F, int S, int W) {
+    const int channel_groups = (F + kChannelsPerCta - 1) / kChannelsPerCta;
+    // windows per CTA: short windows share a CTA's ramp, as long as the launch fills the GPU
+    int run = std::max(1, std::min(kMaxRun, kRunSpectra / S));
+    while (run > 1 && static_cast<long long>(channel_groups) * ((W + run - 1) / run) < kWantedCtas) run /= 2;
+    const bool runs = S <= kShortWindow;
+    const size_t smem = (runs ? 8 * ring_depth<A>() * 16 * A : 0) + 8 * 2 * A * sizeof(uint32_t) +
+                        run * A * sizeof(double) +
+                        (intensity != nullptr ? 2 * kStageBlocks * 16 * kChannelsPerCta * sizeof(float) : 0);
+    auto kernel = runs ? tracker_stream_kernel<A, true> : tracker_stream_kernel<A, false>;
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (err != cudaSuccess) return cuda_status(err, "tracker_stream_kernel smem attribute");
+    const dim3 grid(static_cast<unsigned>((W + run - 1) / run), static_cast<unsigned>(channel_groups));
+    kernel<<<grid, kChannelsPerCta * 32, smem, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S, W, run);
+    return cuda_status(cudaGetLastError(), "tracker_stream_kernel launch");
 }
 
 }  // namespace
@@ -178,28 +366,15 @@ bf_status launch_tracker_stream(cudaStream_t stream, const uint8_t* v, const flo
     if (W > 0x7fffffffull || d.n_time > 0x7fffffffull) {
         return set_error(BF_ERR_OVERFLOW, "CUDA tracker grid exceeds the supported size");
     }
-    const dim3 grid(static_cast<unsigned>(W),
-                    static_cast<unsigned>((d.n_freq + kChannelsPerCta - 1) / kChannelsPerCta));
-    const dim3 block(kChannelsPerCta * 32);
     const int T = static_cast<int>(d.n_time), F = static_cast<int>(d.n_freq);
-    const int S = static_cast<int>(spectra);
+    const int S = static_cast<int>(std::min<uint64_t>(spectra, d.n_time)), w = static_cast<int>(W);
     switch (d.n_ant) {
-        case 32:
-            tracker_stream_kernel<32><<<grid, block, 0, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S);
-            break;
-        case 64:
-            tracker_stream_kernel<64><<<grid, block, 0, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S);
-            break;
-        case 128:
-            tracker_stream_kernel<128><<<grid, block, 0, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S);
-            break;
-        case 256:
-            tracker_stream_kernel<256><<<grid, block, 0, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S);
-            break;
-        default:
-            return set_error(BF_ERR_INVALID_ARGUMENT, "n_ant must be 32, 64, 128, or 256");
+        case 32: return launch_stream<32>(stream, v, pos, k, dirs, intensity, integrated, T, F, S, w);
+        case 64: return launch_stream<64>(stream, v, pos, k, dirs, intensity, integrated, T, F, S, w);
+        case 128: return launch_stream<128>(stream, v, pos, k, dirs, intensity, integrated, T, F, S, w);
+        case 256: return launch_stream<256>(stream, v, pos, k, dirs, intensity, integrated, T, F, S, w);
+        default: return set_error(BF_ERR_INVALID_ARGUMENT, "n_ant must be 32, 64, 128, or 256");
     }
-    return cuda_status(cudaGetLastError(), "tracker_stream_kernel launch");
 }
 
 }  // namespace bf

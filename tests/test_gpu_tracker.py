@@ -82,3 +82,19 @@ def test_mode1_integrated_only_and_point_source(cuda, orc, ref):
     assert np.allclose(integ, exp_w, rtol=1e-5, atol=1e-3)
     # the tracked beam collects (close to) the full coherent power A^2 * 16
     assert float(np.median(exp)) > 0.5 * A * A * 16
+
+
+@pytest.mark.parametrize("A,T,S", [(32, 1003, 1), (32, 7005, 7), (32, 950, 16), (64, 530, 17), (64, 200, 64),
+                                   (64, 200, 65), (64, 161, 33), (128, 130, 129), (256, 37, 12)])
+@pytest.mark.parametrize("outputs", ["both", "integrated"])
+def test_mode1_window_edges(cuda, orc, A, T, S, outputs):
+    """Both forms of the streaming kernel (windows up to 64 spectra in runs of
+    up to 16 per CTA, longer ones one per CTA) at block, run and stage edges,
+    with a partial last window; the tolerance is the file's."""
+    from beamform_project_b200 import api
+    pos, freq, dirs, v, ref = _case(orc, api, T, A, S, seed=T + S)
+    inten, integ = _run(cuda, api, 1, v, pos, freq, dirs, T, A, S, want_int=outputs == "both")
+    if inten is not None:
+        assert np.all(np.abs(inten.astype(np.float64) - ref) <= 1e-3 + 1e-5 * np.abs(ref))
+    exp64 = orc.integrate(ref[..., None], T, F, 1, S)[..., 0].astype(np.float64)
+    assert np.all(np.abs(integ - exp64) <= 1e-3 + 1e-5 * np.abs(exp64))
