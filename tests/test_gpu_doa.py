@@ -314,3 +314,21 @@ def test_adaptive_tracker_takes_the_grid_maximum(cuda, orc, G, M, capon):
         assert np.array_equal(lm[cell], got[w, :2])
         assert p[cell] >= p.max() * (1 - 1e-6)
         centre = got[w, :2]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("A", [32, 64])
+def test_covariance_at_its_least_alignment(cuda, orc, A):
+    """The covariance may start at any multiple of 8 bytes: the wide stores
+    are for 16-byte aligned buffers only."""
+    from beamform_project_b200 import api
+    torch = cuda
+    K, B = 128, 3
+    v = random_voltage(K * B, F, A, seed=A)
+    n = B * F * A * A * 2
+    buf = torch.full((n + 4,), 77, dtype=torch.int32, device="cuda")
+    out = buf[2:2 + n]
+    assert out.data_ptr() % 16 == 8
+    api.doa_covariance_i32(None, torch.from_numpy(v).cuda(), out, api.Dimensions(K * B, F, A, 1), K)
+    assert np.array_equal(out.cpu().numpy().reshape(B, F, A, A, 2).astype(np.int64), orc.covariance_blocks(v, K))
+    assert buf[:2].tolist() == [77, 77] and buf[2 + n:].tolist() == [77, 77]
