@@ -34,9 +34,13 @@
 // 16 x 16 grid of 8 elements, 1 us of the FP64 pipe) is short, so the work is
 // spread thin (192 CTAs where 48 left two thirds of the SMs idle) and the
 // selection rides in the same launch and in all threads of its CTA.
+// A level's matrices do not depend on the level before, so its CTAs come up
+// early (programmatic dependent launch) and copy them to shared memory while
+// the one before finishes.
 // Measured, 32 windows of 256 spectra, 64 antennas, 8 elements, 16 x 16 grid,
-// 2 refinements: 12.8 us per launch, 96 launches (21 us, and 27 us for a
-// selection kernel by one thread after each); the whole call 5.42 -> 1.92 ms.
+// 2 refinements, the whole call: 5.42 ms with a selection kernel of one
+// thread behind each level, 1.77 ms with the selection in the same launch,
+// 1.35 ms with the matrices copied ahead.
 #include "bf_internal.cuh"
 #include "tracker_common.cuh"
 
@@ -220,20 +224,43 @@ template <int M>
 __global__ void __launch_bounds__(kLevelThreads) doa_level_kernel(TrackParams p, int b, float2* __restrict points,
                                                                   SearchState* __restrict state,
                                                                   double* __restrict partial, SelectParams q) {
-    extern __shared__ float pw_large[];  // powers of grids above kMaxDirect points
+    constexpr int U = M * (M + 1) / 2;   // upper triangle incl. diagonal
+    extern __shared__ Cd xs[];           // [kChanGroup][U], then the powers of grids above kMaxDirect points
+    float* pw_large = reinterpret_cast<float*>(xs + kChanGroup * U);
     __shared__ float pw_small[kMaxDirect];
     __shared__ double red[kChanGroup][kPointTile];
     __shared__ double red_w[8][kPointTile];
     __shared__ int s_last;
-    const int n_points = state->n_points;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int pl = lane & 7, cl = lane >> 3;
     const int pt = blockIdx.x * kPointTile + pl;
     const int group = blockIdx.y;
+    // Up to the wait for the level before, a CTA touches only what the fold
+    // wrote: the triangles of its warps' eight channels, all loads in flight
+    // at once.  Once past it, it lets the next level's CTAs come up.
+#pragma unroll 1
+    for (int i = 0; i < kChanGroup / 8; ++i) {
+        const int c = 4 * warp + (i & 3) + 32 * (i >> 2), f = group * kChanGroup + c;
+        if (f >= p.n_freq) continue;
+        const Cd* X = (p.capon ? p.Q : p.S) + (static_cast<size_t>(b) * p.n_freq + f) * M * M;
+        for (int e = lane; e < M * M; e += 32) {
+            const int r = e / M, k = e % M;
+            if (k < r) continue;
+            const uint32_t dst = static_cast<uint32_t>(
+                __cvta_generic_to_shared(xs + c * U + r * M - r * (r - 1) / 2 + (k - r)));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(X + e) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int n_points = state->n_points;
     const float2 lm = pt < n_points ? points[pt] : make_float2(0.f, 0.f);
     const double l = lm.x, m = lm.y;
     // n as direction_from_lm forms it (float), for arrays with z != 0
     const double n = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(lm.x, lm.x), __fmul_rn(lm.y, lm.y))));
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
 #pragma unroll 1
     for (int c = 4 * warp + cl; c < kChanGroup; c += 32) {
         const int f = group * kChanGroup + c;
@@ -250,15 +277,16 @@ __global__ void __launch_bounds__(kLevelThreads) doa_level_kernel(TrackParams p,
                 a[i] = Cd{static_cast<double>(w.x), -static_cast<double>(w.y)};  // exp(-i phase)
                 mag[i] = a[i].re * a[i].re + a[i].im * a[i].im;
             }
-            const Cd* X = (p.capon ? p.Q : p.S) + cell * M * M;
+            const Cd* X = xs + c * U;
             double diag = 0.0, off = 0.0;
+            int t = 0;
 #pragma unroll
             for (int r = 0; r < M; ++r) {
-                diag += X[r * M + r].re * mag[r];
+                diag += X[t++].re * mag[r];
                 double tr = 0.0, ti = 0.0;
 #pragma unroll
                 for (int e = r + 1; e < M; ++e) {
-                    const Cd x = X[r * M + e];
+                    const Cd x = X[t++];
                     tr += x.re * a[e].re - x.im * a[e].im;
                     ti += x.re * a[e].im + x.im * a[e].re;
                 }
@@ -313,9 +341,26 @@ bf_status launch_level(int m, cudaStream_t stream, const TrackParams& p, int b, 
         if (m != M) return launch_level<M + 1>(m, stream, p, b, points, st, partial, n_points, q);
         const dim3 grid(static_cast<unsigned>((n_points + kPointTile - 1) / kPointTile),
                         static_cast<unsigned>(q.n_groups));
-        const size_t smem = n_points > kMaxDirect ? n_points * sizeof(float) : 0;
-        doa_level_kernel<M><<<grid, kLevelThreads, smem, stream>>>(p, b, points, st, partial, q);
-        return cuda_status(cudaGetLastError(), "doa_level_kernel launch");
+        const int smem = kChanGroup * M * (M + 1) / 2 * static_cast<int>(sizeof(Cd)) +
+                         (n_points > kMaxDirect ? n_points * static_cast<int>(sizeof(float)) : 0);
+        const cudaError_t err =
+            cudaFuncSetAttribute(doa_level_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err != cudaSuccess) return cuda_status(err, "doa_level_kernel smem attribute");
+        // each level but the first comes up while the one before it runs
+        // (programmatic dependent launch): the first waits for the fold, and
+        // none of the others starts before it
+        cudaLaunchAttribute overlap{};
+        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        overlap.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = dim3(kLevelThreads);
+        cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+        cfg.stream = stream;
+        cfg.attrs = &overlap;
+        cfg.numAttrs = b > 0 || q.level > 0 ? 1 : 0;
+        return cuda_status(cudaLaunchKernelEx(&cfg, doa_level_kernel<M>, p, b, points, st, partial, q),
+                           "doa_level_kernel launch");
     }
 }
 
