@@ -25,24 +25,26 @@
 // precision.  Grid construction, clamping and interpolation are float32 with
 // the reference's operation order.
 //
-// One launch per window and level.  A CTA takes 8 points and a group of 64
-// channels (lane = one of 8 points, one of 4 channels), writes one partial
-// sum per (point, group), and the CTA that finishes last adds the groups in
-// order, takes the argmax and writes the next level's points, or the
-// window's direction and the next window's grid.  What bounds it: the chain
-// of windows and levels, each a launch whose work (2e7 FP64 operations for a
-// 16 x 16 grid of 8 elements, 1 us of the FP64 pipe) is short, so the work is
-// spread thin (192 CTAs where 48 left two thirds of the SMs idle) and the
-// selection rides in the same launch and in all threads of its CTA.
-// A level's matrices do not depend on the level before, so its CTAs come up
-// early (programmatic dependent launch) and copy them to shared memory while
-// the one before finishes.
+// One launch per window, in clusters of one CTA per group of 64 channels.  A
+// cluster evaluates 16 coarse points, adds the groups' sums in order through
+// distributed shared memory and writes their powers; the cluster that
+// finishes last selects the maximum and runs the refinements by itself, its
+// CTAs exchanging sums and each selecting alike, so a refinement costs one
+// cluster barrier instead of a launch.  A window's matrices do not depend on
+// the window before, so its CTAs come up early (programmatic dependent
+// launch) and copy their channels' triangles to shared memory while that one
+// finishes; the refinements use the same copies.
+// What bounds it: the chain of windows and levels.  A level's work is short
+// (2e7 FP64 operations for a 16 x 16 grid of 8 elements, 1 us of the FP64
+// pipe), its exchanges are latency.
 // Measured, 32 windows of 256 spectra, 64 antennas, 8 elements, 16 x 16 grid,
-// 2 refinements, the whole call: 5.42 ms with a selection kernel of one
-// thread behind each level, 1.77 ms with the selection in the same launch,
-// 1.35 ms with the matrices copied ahead.
+// 2 refinements, the whole call: 1.03 ms, 19 us of it per window (1.35 ms
+// with a launch per level, 5.42 ms with a one-thread selection kernel behind
+// each).
 #include "bf_internal.cuh"
 #include "tracker_common.cuh"
+
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
@@ -61,10 +63,9 @@ struct Cd {
 
 // Search state between launches (device memory).
 struct SearchState {
-    float cl, cm;          // running centre (l, m)
-    float half_l, half_m;  // refinement half-pitch of the current level
-    int n_points;          // points of the current level
-    unsigned done;         // CTAs of the running level kernel that have written their sums
+    float cl, cm;          // the previous window's estimate: centre of the coarse grid
+    unsigned done;         // clusters of the running launch that have written their powers
+    unsigned pad[3];
 };
 
 struct TrackParams {
@@ -106,38 +107,27 @@ __device__ __forceinline__ float2 coarse_point(int i, float cl, float cm, int G,
                       __fadd_rn(start_m, __fmul_rn(static_cast<float>(v), step_m)));
 }
 
-constexpr int kLevelThreads = 256;
-constexpr int kPointTile = 8;        // points per CTA
-constexpr int kMaxDirect = 256;      // points whose powers fit the fixed shared array
+constexpr int kCoarseTile = 16;      // coarse points per cluster
+constexpr int kFine = 9;             // candidates of a refinement
+constexpr int kSearchThreads = kFine * kChanGroup;
+constexpr int kMaxGroups = 8;        // CTAs per cluster (a portable cluster)
 
-// What a level's selection needs beside the powers.
-struct SelectParams {
-    int n_groups, level, levels, G;
+struct SearchParams {
+    int levels, G;
     float fov_l, fov_m;
     int interp;
     float* dir_out;
-    int last_window;
 };
 
-// By every thread of the last CTA: the level's powers in float, as the
-// reference compares and interpolates them, their first maximum, and the next
-// level or window.  pw holds the powers (shared memory).
-__device__ __forceinline__ void select_level(const double* __restrict partial, float2* __restrict points,
-                                             SearchState* __restrict st, const SelectParams& q, int n,
-                                             float* __restrict pw) {
-    constexpr int kWarps = kLevelThreads / 32;
-    __shared__ float best_v[kWarps];
-    __shared__ int best_i[kWarps];
-    __shared__ float next[4];  // centre and half-pitches of the next level
-    const int tid = threadIdx.x, lane = tid & 31;
+// First maximum of pw[0, n) by the CTA's threads: strict > over increasing
+// index; n when every power is -inf or NaN.  Returned to thread 0.
+__device__ __forceinline__ int first_maximum(const float* __restrict pw, int n, float* best_v, int* best_i) {
+    const int tid = threadIdx.x;
     float bv = -INFINITY;
     int bi = n;
-    for (int i = tid; i < n; i += kLevelThreads) {
-        double s = 0.0;
-        for (int g = 0; g < q.n_groups; ++g) s += __ldcg(partial + static_cast<size_t>(g) * kMaxPoints + i);
-        const float x = static_cast<float>(s);
-        pw[i] = x;
-        if (x > bv) { bv = x; bi = i; }  // first maximum: strict > over increasing index
+    for (int i = tid; i < n; i += kSearchThreads) {
+        const float x = __ldcg(pw + i);
+        if (x > bv) { bv = x; bi = i; }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -145,222 +135,261 @@ __device__ __forceinline__ void select_level(const double* __restrict partial, f
         const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
         if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
-    if (lane == 0) {
+    if ((tid & 31) == 0) {
         best_v[tid >> 5] = bv;
         best_i[tid >> 5] = bi;
     }
     __syncthreads();
     if (tid == 0) {
-        for (int w = 1; w < kWarps; ++w) {
+        for (int w = 1; w < kSearchThreads / 32; ++w) {
             if (best_v[w] > bv || (best_v[w] == bv && best_i[w] < bi)) { bv = best_v[w]; bi = best_i[w]; }
         }
-        if (bi >= n) bi = 0;  // every power NaN-free and -inf: the first cell, as the reference
-        const float2 best = points[bi];
-        float cl = best.x, cm = best.y, half_l = st->half_l, half_m = st->half_m;
-        if (q.level == 0) {
+    }
+    return bi;
+}
+
+// The search of window b: the coarse grid by every cluster, the rest by the
+// cluster that finishes it.  Sums over channels keep one order at every
+// level: within a group channels w, w + 8, ... first, then w = 0 .. 7, then
+// the groups.
+template <int M>
+__global__ void __launch_bounds__(kSearchThreads, 1)
+doa_search_kernel(TrackParams p, int b, SearchState* __restrict st, float* __restrict powers, SearchParams q) {
+    namespace cg = cooperative_groups;
+    constexpr int U = M * (M + 1) / 2;   // upper triangle incl. diagonal
+    extern __shared__ Cd xs[];           // [kChanGroup][U]
+    __shared__ double kw_s[kChanGroup];
+    __shared__ int ok_s[kChanGroup];
+    __shared__ double delay_s[kCoarseTile][M];
+    __shared__ double red[kChanGroup][kCoarseTile], red_w[8][kCoarseTile];
+    __shared__ double part[2][kMaxGroups][kCoarseTile];  // the groups' sums, by level parity
+    __shared__ float best_v[kSearchThreads / 32];
+    __shared__ int best_i[kSearchThreads / 32];
+    __shared__ float fine_pw[kFine];
+    __shared__ float centre[4];          // running centre and half-pitches
+    __shared__ int s_last;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int tid = threadIdx.x, group = static_cast<int>(cluster.block_rank());
+    const int n_groups = static_cast<int>(gridDim.y);
+    const int f0 = group * kChanGroup, nf = min(kChanGroup, p.n_freq - f0);
+    // Up to the wait for the window before, a CTA touches only what the fold
+    // wrote and the caller's arrays.
+    const Cd* X0 = (p.capon ? p.Q : p.S) + (static_cast<size_t>(b) * p.n_freq + f0) * M * M;
+    for (int i = tid; i < nf * M * M; i += kSearchThreads) {
+        const int c = i / (M * M), e = i % (M * M), r = e / M, k = e % M;
+        if (k < r) continue;
+        const uint32_t dst =
+            static_cast<uint32_t>(__cvta_generic_to_shared(xs + c * U + r * M - r * (r - 1) / 2 + (k - r)));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(X0 + i) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (tid < nf) {
+        kw_s[tid] = p.kw[f0 + tid];
+        ok_s[tid] = p.ok[static_cast<size_t>(b) * p.n_freq + f0 + tid];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    // Powers of the group's channels at np points, summed over them into
+    // red_w's column sums: thread pt < np returns the group's sum.
+    auto point_sum = [&](int np, auto point) -> double {
+        for (int i = tid; i < np * M; i += kSearchThreads) {
+            const float2 lm = point(i / M);
+            // n as direction_from_lm forms it (float), for arrays with z != 0
+            const float n = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(lm.x, lm.x), __fmul_rn(lm.y, lm.y))));
+            delay_s[i / M][i % M] = trk::steering_delay(p.pos, i % M, lm.x, lm.y, n);
+        }
+        __syncthreads();
+        const int pt = tid % np, per = kSearchThreads / np;
+#pragma unroll 1
+        for (int c = tid / np; c < kChanGroup && tid < per * np; c += per) {
+            double pw = 0.0;
+            if (c < nf) {
+                const double k = kw_s[c];
+                Cd a[M];
+                double mag[M];
+#pragma unroll
+                for (int i = 0; i < M; ++i) {
+                    const float2 w = trk::steering_from_delay(k, delay_s[pt][i]);
+                    a[i] = Cd{static_cast<double>(w.x), -static_cast<double>(w.y)};  // exp(-i phase)
+                    mag[i] = a[i].re * a[i].re + a[i].im * a[i].im;
+                }
+                const Cd* X = xs + c * U;
+                double diag = 0.0, off = 0.0;
+                int t = 0;
+#pragma unroll
+                for (int r = 0; r < M; ++r) {
+                    diag += X[t++].re * mag[r];
+                    double tr = 0.0, ti = 0.0;
+#pragma unroll
+                    for (int e = r + 1; e < M; ++e) {
+                        const Cd x = X[t++];
+                        tr += x.re * a[e].re - x.im * a[e].im;
+                        ti += x.re * a[e].im + x.im * a[e].re;
+                    }
+                    off += a[r].re * tr + a[r].im * ti;  // Re(conj(a_r) * (X a)_r upper part)
+                }
+                pw = diag + 2.0 * off;
+                if (p.capon) pw = (ok_s[c] && pw > 0.0) ? 1.0 / pw : 0.0;
+                if (!isfinite(pw)) pw = 0.0;
+            }
+            red[c][pt] = pw;
+        }
+        __syncthreads();
+        if (tid < 8 * np) {
+            const int w = tid / np;
+            double acc = 0.0;
+#pragma unroll
+            for (int i = 0; i < kChanGroup / 8; ++i) acc += red[w + 8 * i][tid % np];
+            red_w[w][tid % np] = acc;
+        }
+        __syncthreads();
+        double s = 0.0;
+        if (tid < np) {
+#pragma unroll
+            for (int w = 0; w < 8; ++w) s += red_w[w][tid];
+        }
+        return s;
+    };
+    auto groups_sum = [&](int buf, int pt) {
+        double s = 0.0;
+        for (int g = 0; g < n_groups; ++g) s += part[buf][g][pt];
+        return static_cast<float>(s);  // powers in float, as the reference compares and interpolates them
+    };
+
+    // the coarse grid
+    const float c0_l = st->cl, c0_m = st->cm;
+    const int n_points = q.G * q.G;
+    const int i0 = blockIdx.x * kCoarseTile, np = min(kCoarseTile, n_points - i0);
+    {
+        const double s = point_sum(np, [&](int i) { return coarse_point(i0 + i, c0_l, c0_m, q.G, q.fov_l, q.fov_m); });
+        if (tid < np) *cluster.map_shared_rank(&part[0][group][tid], 0) = s;
+    }
+    cluster.sync();
+    if (group == 0) {
+        if (tid < np) {
+            powers[i0 + tid] = groups_sum(0, tid);
+            __threadfence();
+        }
+        __syncthreads();
+        if (tid == 0) {
+            const int last = atomicAdd(&st->done, 1u) + 1 == gridDim.x;
+            __threadfence();
+            for (int r = 0; r < n_groups; ++r) *cluster.map_shared_rank(&s_last, r) = last;
+        }
+    }
+    cluster.sync();
+    if (!s_last) return;
+
+    const float step_l = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_l), static_cast<float>(q.G - 1));
+    const float step_m = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_m), static_cast<float>(q.G - 1));
+    {
+        // every CTA of the cluster selects for itself, alike
+        int bi = first_maximum(powers, n_points, best_v, best_i);
+        if (tid == 0) {
+            if (bi >= n_points) bi = 0;  // no power above -inf: the first cell, as the reference
+            float2 c = coarse_point(bi, c0_l, c0_m, q.G, q.fov_l, q.fov_m);
             if (q.levels == 0 && q.interp) {
                 const int u = bi % q.G, v = bi / q.G;
                 auto at = [&](int du, int dv) -> float {
                     const int uu = u + du, vv = v + dv;
-                    return (uu < 0 || uu >= q.G || vv < 0 || vv >= q.G) ? 0.0f : pw[vv * q.G + uu];
+                    return (uu < 0 || uu >= q.G || vv < 0 || vv >= q.G) ? 0.0f : __ldcg(powers + vv * q.G + uu);
                 };
-                const float pc = pw[bi];
+                const float pc = at(0, 0);
                 const float du = interp_offset(pc, at(1, 0), at(-1, 0));
                 const float dv = interp_offset(pc, at(0, 1), at(0, -1));
-                const float step_l = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_l), static_cast<float>(q.G - 1));
-                const float step_m = q.G == 1 ? 0.0f : __fdiv_rn(__fmul_rn(2.0f, q.fov_m), static_cast<float>(q.G - 1));
-                const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, step_l)), __fadd_rn(cm, __fmul_rn(dv, step_m)));
-                cl = c.x;
-                cm = c.y;
+                c = clamp_disk(__fadd_rn(c.x, __fmul_rn(du, step_l)), __fadd_rn(c.y, __fmul_rn(dv, step_m)));
             }
-            half_l = __fdiv_rn(q.fov_l, static_cast<float>(q.G));
-            half_m = __fdiv_rn(q.fov_m, static_cast<float>(q.G));
-        } else if (q.interp) {
-            // the candidates' centre row and column, whichever candidate won
-            const float du = interp_offset(pw[4], pw[5], pw[3]);
-            const float dv = interp_offset(pw[4], pw[7], pw[1]);
-            const float2 c = clamp_disk(__fadd_rn(cl, __fmul_rn(du, half_l)), __fadd_rn(cm, __fmul_rn(dv, half_m)));
-            cl = c.x;
-            cm = c.y;
+            centre[0] = c.x;
+            centre[1] = c.y;
+            centre[2] = __fmul_rn(__fdiv_rn(q.fov_l, static_cast<float>(q.G)), 0.5f);
+            centre[3] = __fmul_rn(__fdiv_rn(q.fov_m, static_cast<float>(q.G)), 0.5f);
         }
-        if (q.level < q.levels) {
-            half_l = __fmul_rn(half_l, 0.5f);
-            half_m = __fmul_rn(half_m, 0.5f);
-        } else {
-            // the window's direction (direction_from_lm)
-            q.dir_out[0] = cl;
-            q.dir_out[1] = cm;
-            q.dir_out[2] = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(cl, cl), __fmul_rn(cm, cm))));
+        __syncthreads();
+    }
+    for (int level = 1; level <= q.levels; ++level) {
+        const int buf = level & 1;
+        auto candidate = [&](int i) {
+            const float du = static_cast<float>(i % 3 - 1), dv = static_cast<float>(i / 3 - 1);
+            return clamp_disk(__fadd_rn(centre[0], __fmul_rn(du, centre[2])),
+                              __fadd_rn(centre[1], __fmul_rn(dv, centre[3])));
+        };
+        const double s = point_sum(kFine, candidate);
+        if (tid < kFine) {
+            for (int r = 0; r < n_groups; ++r) *cluster.map_shared_rank(&part[buf][group][tid], r) = s;
         }
+        cluster.sync();
+        if (tid < kFine) fine_pw[tid] = groups_sum(buf, tid);
+        __syncthreads();
+        if (tid == 0) {
+            float bv = -INFINITY;
+            int bi = kFine;
+            for (int i = 0; i < kFine; ++i) {
+                if (fine_pw[i] > bv) { bv = fine_pw[i]; bi = i; }
+            }
+            float2 c = candidate(bi >= kFine ? 0 : bi);
+            if (q.interp) {
+                // the candidates' centre row and column, whichever candidate won
+                const float du = interp_offset(fine_pw[4], fine_pw[5], fine_pw[3]);
+                const float dv = interp_offset(fine_pw[4], fine_pw[7], fine_pw[1]);
+                c = clamp_disk(__fadd_rn(c.x, __fmul_rn(du, centre[2])), __fadd_rn(c.y, __fmul_rn(dv, centre[3])));
+            }
+            centre[0] = c.x;
+            centre[1] = c.y;
+            centre[2] = __fmul_rn(centre[2], 0.5f);
+            centre[3] = __fmul_rn(centre[3], 0.5f);
+        }
+        __syncthreads();
+    }
+    if (group == 0 && tid == 0) {
+        // the window's direction (direction_from_lm), centre of the next window's grid
+        const float cl = centre[0], cm = centre[1];
+        q.dir_out[0] = cl;
+        q.dir_out[1] = cm;
+        q.dir_out[2] = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(cl, cl), __fmul_rn(cm, cm))));
         st->cl = cl;
         st->cm = cm;
-        st->half_l = half_l;
-        st->half_m = half_m;
-        st->n_points = q.level < q.levels ? 9 : q.G * q.G;
-        st->done = 0;
-        next[0] = cl;
-        next[1] = cm;
-        next[2] = half_l;
-        next[3] = half_m;
-    }
-    __syncthreads();
-    if (q.level < q.levels) {
-        if (tid < 9) {
-            const float du = static_cast<float>(tid % 3 - 1), dv = static_cast<float>(tid / 3 - 1);
-            points[tid] = clamp_disk(__fadd_rn(next[0], __fmul_rn(du, next[2])),
-                                     __fadd_rn(next[1], __fmul_rn(dv, next[3])));
-        }
-    } else if (!q.last_window) {
-        for (int i = tid; i < q.G * q.G; i += kLevelThreads) {
-            points[i] = coarse_point(i, next[0], next[1], q.G, q.fov_l, q.fov_m);
-        }
-    }
-}
-
-// Bartlett or Capon power of window `b` at the points, summed over each
-// 64-channel group (partial[group][point]: channels w, w + 8, ... of the
-// group first, then w = 0 .. 7), and the selection by the last CTA.
-template <int M>
-__global__ void __launch_bounds__(kLevelThreads) doa_level_kernel(TrackParams p, int b, float2* __restrict points,
-                                                                  SearchState* __restrict state,
-                                                                  double* __restrict partial, SelectParams q) {
-    constexpr int U = M * (M + 1) / 2;   // upper triangle incl. diagonal
-    extern __shared__ Cd xs[];           // [kChanGroup][U], then the powers of grids above kMaxDirect points
-    float* pw_large = reinterpret_cast<float*>(xs + kChanGroup * U);
-    __shared__ float pw_small[kMaxDirect];
-    __shared__ double red[kChanGroup][kPointTile];
-    __shared__ double red_w[8][kPointTile];
-    __shared__ int s_last;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int pl = lane & 7, cl = lane >> 3;
-    const int pt = blockIdx.x * kPointTile + pl;
-    const int group = blockIdx.y;
-    // Up to the wait for the level before, a CTA touches only what the fold
-    // wrote: the triangles of its warps' eight channels, all loads in flight
-    // at once.  Once past it, it lets the next level's CTAs come up.
-#pragma unroll 1
-    for (int i = 0; i < kChanGroup / 8; ++i) {
-        const int c = 4 * warp + (i & 3) + 32 * (i >> 2), f = group * kChanGroup + c;
-        if (f >= p.n_freq) continue;
-        const Cd* X = (p.capon ? p.Q : p.S) + (static_cast<size_t>(b) * p.n_freq + f) * M * M;
-        for (int e = lane; e < M * M; e += 32) {
-            const int r = e / M, k = e % M;
-            if (k < r) continue;
-            const uint32_t dst = static_cast<uint32_t>(
-                __cvta_generic_to_shared(xs + c * U + r * M - r * (r - 1) / 2 + (k - r)));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(X + e) : "memory");
-        }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int n_points = state->n_points;
-    const float2 lm = pt < n_points ? points[pt] : make_float2(0.f, 0.f);
-    const double l = lm.x, m = lm.y;
-    // n as direction_from_lm forms it (float), for arrays with z != 0
-    const double n = __fsqrt_rn(__fsub_rn(1.0f, __fadd_rn(__fmul_rn(lm.x, lm.x), __fmul_rn(lm.y, lm.y))));
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp();
-#pragma unroll 1
-    for (int c = 4 * warp + cl; c < kChanGroup; c += 32) {
-        const int f = group * kChanGroup + c;
-        double pw = 0.0;
-        if (f < p.n_freq && pt < n_points) {
-            const size_t cell = static_cast<size_t>(b) * p.n_freq + f;
-            const double k = p.kw[f];
-            Cd a[M];
-            double mag[M];
-#pragma unroll
-            for (int i = 0; i < M; ++i) {
-                const double delay = trk::steering_delay(p.pos, i, l, m, n);
-                const float2 w = trk::steering_from_delay(k, delay);
-                a[i] = Cd{static_cast<double>(w.x), -static_cast<double>(w.y)};  // exp(-i phase)
-                mag[i] = a[i].re * a[i].re + a[i].im * a[i].im;
-            }
-            const Cd* X = xs + c * U;
-            double diag = 0.0, off = 0.0;
-            int t = 0;
-#pragma unroll
-            for (int r = 0; r < M; ++r) {
-                diag += X[t++].re * mag[r];
-                double tr = 0.0, ti = 0.0;
-#pragma unroll
-                for (int e = r + 1; e < M; ++e) {
-                    const Cd x = X[t++];
-                    tr += x.re * a[e].re - x.im * a[e].im;
-                    ti += x.re * a[e].im + x.im * a[e].re;
-                }
-                off += a[r].re * tr + a[r].im * ti;  // Re(conj(a_r) * (X a)_r upper part)
-            }
-            pw = diag + 2.0 * off;
-            if (p.capon) pw = (p.ok[cell] && pw > 0.0) ? 1.0 / pw : 0.0;
-            if (!isfinite(pw)) pw = 0.0;
-        }
-        red[c][pl] = pw;
-    }
-    __syncthreads();
-    if (threadIdx.x < 8 * kPointTile) {
-        const int w = threadIdx.x >> 3;
-        double acc = 0.0;
-#pragma unroll
-        for (int i = 0; i < kChanGroup / 8; ++i) acc += red[w + 8 * i][threadIdx.x & 7];
-        red_w[w][threadIdx.x & 7] = acc;
-    }
-    __syncthreads();
-    if (threadIdx.x < kPointTile && blockIdx.x * kPointTile + threadIdx.x < n_points) {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) s += red_w[w][threadIdx.x];
-        partial[static_cast<size_t>(group) * kMaxPoints + blockIdx.x * kPointTile + threadIdx.x] = s;
-        __threadfence();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_last = atomicAdd(&state->done, 1u) + 1 == gridDim.x * gridDim.y;
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_last) select_level(partial, points, state, q, n_points, n_points <= kMaxDirect ? pw_small : pw_large);
-}
-
-__global__ void doa_track_init_kernel(SearchState* st, float2* points, float l0, float m0, int G, float fov_l,
-                                      float fov_m) {
-    for (int i = threadIdx.x; i < G * G; i += blockDim.x) points[i] = coarse_point(i, l0, m0, G, fov_l, fov_m);
-    if (threadIdx.x == 0) {
-        st->n_points = G * G;
         st->done = 0;
     }
 }
 
+__global__ void doa_track_init_kernel(SearchState* st, float l0, float m0) {
+    st->cl = l0;
+    st->cm = m0;
+    st->done = 0;
+}
+
 template <int M>
-bf_status launch_level(int m, cudaStream_t stream, const TrackParams& p, int b, float2* points, SearchState* st,
-                       double* partial, int n_points, const SelectParams& q) {
+bf_status launch_search(int m, cudaStream_t stream, const TrackParams& p, int b, SearchState* st, float* powers,
+                        int n_groups, const SearchParams& q) {
     if constexpr (M > kMaxM) {
         return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 16 elements after smoothing");
     } else {
-        if (m != M) return launch_level<M + 1>(m, stream, p, b, points, st, partial, n_points, q);
-        const dim3 grid(static_cast<unsigned>((n_points + kPointTile - 1) / kPointTile),
-                        static_cast<unsigned>(q.n_groups));
-        const int smem = kChanGroup * M * (M + 1) / 2 * static_cast<int>(sizeof(Cd)) +
-                         (n_points > kMaxDirect ? n_points * static_cast<int>(sizeof(float)) : 0);
+        if (m != M) return launch_search<M + 1>(m, stream, p, b, st, powers, n_groups, q);
+        const int smem = kChanGroup * M * (M + 1) / 2 * static_cast<int>(sizeof(Cd));
         const cudaError_t err =
-            cudaFuncSetAttribute(doa_level_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) return cuda_status(err, "doa_level_kernel smem attribute");
-        // each level but the first comes up while the one before it runs
-        // (programmatic dependent launch): the first waits for the fold, and
-        // none of the others starts before it
-        cudaLaunchAttribute overlap{};
-        overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        overlap.val.programmaticStreamSerializationAllowed = 1;
+            cudaFuncSetAttribute(doa_search_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (err != cudaSuccess) return cuda_status(err, "doa_search_kernel smem attribute");
+        cudaLaunchAttribute attrs[2] = {};
+        attrs[0].id = cudaLaunchAttributeClusterDimension;
+        attrs[0].val.clusterDim.x = 1;
+        attrs[0].val.clusterDim.y = static_cast<unsigned>(n_groups);
+        attrs[0].val.clusterDim.z = 1;
+        // each window but the first comes up while the one before it runs: the
+        // first waits for the fold, and none of the others starts before it
+        attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[1].val.programmaticStreamSerializationAllowed = 1;
         cudaLaunchConfig_t cfg{};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(kLevelThreads);
+        cfg.gridDim = dim3(static_cast<unsigned>((q.G * q.G + kCoarseTile - 1) / kCoarseTile),
+                           static_cast<unsigned>(n_groups));
+        cfg.blockDim = dim3(kSearchThreads);
         cfg.dynamicSmemBytes = static_cast<size_t>(smem);
         cfg.stream = stream;
-        cfg.attrs = &overlap;
-        cfg.numAttrs = b > 0 || q.level > 0 ? 1 : 0;
-        return cuda_status(cudaLaunchKernelEx(&cfg, doa_level_kernel<M>, p, b, points, st, partial, q),
-                           "doa_level_kernel launch");
+        cfg.attrs = attrs;
+        cfg.numAttrs = b > 0 ? 2 : 1;
+        return cuda_status(cudaLaunchKernelEx(&cfg, doa_search_kernel<M>, p, b, st, powers, q),
+                           "doa_search_kernel launch");
     }
 }
 
@@ -371,10 +400,8 @@ uint64_t align256(uint64_t x) { return (x + 255) / 256 * 256; }
 uint64_t doa_track_workspace_bytes(const bf_dims& d, uint64_t block_len, uint64_t subarray) {
     const uint64_t B = d.n_time / block_len, F = d.n_freq, A = d.n_ant;
     const uint64_t M = (subarray > 0 && subarray < A) ? subarray : A;
-    const uint64_t groups = (F + kChanGroup - 1) / kChanGroup;
     return align256(B * F * A * A * 2 * sizeof(int32_t)) + align256(doa_fold_bytes(B * F, M)) +
-           align256(kMaxPoints * sizeof(float2)) + align256(groups * kMaxPoints * sizeof(double)) +
-           align256(sizeof(SearchState));
+           align256(kMaxPoints * sizeof(float)) + align256(sizeof(SearchState));
 }
 
 bf_status launch_doa_track(cudaStream_t stream, const uint8_t* v, const float* pos, const double* kw,
@@ -385,15 +412,14 @@ bf_status launch_doa_track(cudaStream_t stream, const uint8_t* v, const float* p
     const int M = static_cast<int>((c.subarray > 0 && c.subarray < A) ? c.subarray : A);
     if (M > kMaxM) return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 16 elements after smoothing");
     const uint64_t groups = (F + kChanGroup - 1) / kChanGroup;
+    if (groups > kMaxGroups) return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 512 channels");
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     auto* R = reinterpret_cast<int32_t*>(ws);
     ws += align256(static_cast<uint64_t>(B) * F * A * A * 2 * sizeof(int32_t));
     void* fold = ws;
     ws += align256(doa_fold_bytes(static_cast<uint64_t>(B) * F, M));
-    auto* points = reinterpret_cast<float2*>(ws);
-    ws += align256(kMaxPoints * sizeof(float2));
-    auto* partial = reinterpret_cast<double*>(ws);
-    ws += align256(groups * kMaxPoints * sizeof(double));
+    auto* powers = reinterpret_cast<float*>(ws);
+    ws += align256(kMaxPoints * sizeof(float));
     auto* st = reinterpret_cast<SearchState*>(ws);
 
     BF_RETURN_IF(launch_doa_covariance(stream, v, R, d, K));
@@ -408,22 +434,17 @@ bf_status launch_doa_track(cudaStream_t stream, const uint8_t* v, const float* p
     p.n_freq = static_cast<int>(F);
     p.M = M;
     p.capon = c.estimator != 0;
-    const int G = static_cast<int>(c.grid), L = static_cast<int>(c.levels);
-    doa_track_init_kernel<<<1, 256, 0, stream>>>(st, points, c.prior_l, c.prior_m, G, c.fov_l, c.fov_m);
+    doa_track_init_kernel<<<1, 1, 0, stream>>>(st, c.prior_l, c.prior_m);
     BF_RETURN_IF(cuda_status(cudaGetLastError(), "doa_track_init_kernel launch"));
-    SelectParams q{};
-    q.n_groups = static_cast<int>(groups);
-    q.levels = L;
-    q.G = G;
+    SearchParams q{};
+    q.levels = static_cast<int>(c.levels);
+    q.G = static_cast<int>(c.grid);
     q.fov_l = c.fov_l;
     q.fov_m = c.fov_m;
     q.interp = c.interp != 0;
     for (int b = 0; b < B; ++b) {
         q.dir_out = dirs + 3 * b;
-        q.last_window = b + 1 == B;
-        for (q.level = 0; q.level <= L; ++q.level) {
-            BF_RETURN_IF(launch_level<1>(M, stream, p, b, points, st, partial, q.level == 0 ? G * G : 9, q));
-        }
+        BF_RETURN_IF(launch_search<1>(M, stream, p, b, st, powers, static_cast<int>(groups), q));
     }
     if (intensity == nullptr) return BF_OK;
     // emission: the reference-order tracker along each window's estimate
