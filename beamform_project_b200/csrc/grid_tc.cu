@@ -341,8 +341,8 @@ __host__ __device__ constexpr Smem smem_plan(int n_ant, int n_beams_pad, bool se
     // tiles in flight, which the short MMAs of small beam groups need
     s.raw_stages = n_ant == 128 ? kMaxRawStages : 2;
     // window partial sums (S >= 32) or the per-warp power staging of short
-    // windows ([8 warps][16 beams][33] floats), which share the space
-    const uint32_t ring = kRing * 4 * n_beams_pad * 4, staging = (kEpilogueThreads / 32) * 16 * 33 * 4;
+    // windows ([8 warps][32 rows][16 beams] floats), which share the space
+    const uint32_t ring = kRing * 4 * n_beams_pad * 4, staging = (kEpilogueThreads / 32) * 32 * 16 * 4;
     const uint32_t rest = 2 * s.x_bytes + s.raw_stages * s.raw_bytes + (ring > staging ? ring : staging) + 256;
     // A second weight image lets the next channel's weights load while the
     // MMAs of the current one run.  Served units (one window, a few tiles)
@@ -744,7 +744,7 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         constexpr int kHalfLoads = (kLoads + kHalves - 1) / kHalves;
         const int c_begin = half * kHalfLoads;
         const int c_count = min(kHalfLoads, kLoads - c_begin);
-        float* stg = slots + (warp - kEpiFirstWarp) * 528;  // short windows: [16 beams][33]
+        float* stg = slots + (warp - kEpiFirstWarp) * 512;  // short windows: [32 rows][16 beams]
         float acc[kHalfLoads];
 #pragma unroll
         for (int c = 0; c < kHalfLoads; ++c) acc[c] = 0.f;
@@ -762,47 +762,86 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             for (int c = 0; c < kHalfLoads; ++c) acc[c] = 0.f;
         };
         // Short windows (S < 32): every window lies inside one lane quadrant.
-        // The 16 powers of each lane's spectrum go to the staging tile
-        // [16 beams][33] (row pitch 33 floats: the stores of a beam and the
-        // reads of a window both spread over the banks) and each lane sums a
-        // (window, beam) pair of the quadrant, in increasing row order.  wq is
-        // the quadrant's first window; the unit's window length sw and pair
-        // count npairs (16 per window) are set once per unit.
-        auto nwin_of = [](int npairs) { return npairs >> 4; };
-        auto short_windows = [&](const uint32_t (&r)[32], int c, const TcJob& jb, const Unit& un, int wq, int sw,
-                                 int npairs) {
-            float* srow = stg + lane;
+        // Each lane puts the 16 powers of its spectrum into the warp's staging
+        // tile as four 16-byte chunks, chunk j of row r at j ^ (r / 2 % 4) of
+        // the row's 64 bytes (eight rows' stores cover all banks); then a lane
+        // sums two beams of a window in increasing row order (8 byte loads).
+        // What bounds it: shared memory.  At 64 antennas and 128 beams a tile's
+        // MMAs read 196 KB of operands and the powers cross it twice (128 KB),
+        // 2900 clocks of its port against 2180 of MMAs, and two epilogue warps
+        // per scheduler hide little of its latency (4200 clocks per tile, timed
+        // in the kernel).  Measured there, 8000 spectra in windows of 10: 0.457
+        // ms (0.481 with 4-byte stores and loads, addresses formed per sum and a
+        // barrier per tile), of 30 0.547 (0.625); 64 beams in windows of 10 0.300
+        // (0.342).
+        const int s_lane = lane >> 3, b_lane = 2 * (lane & 7);  // window, beams of this lane's sums
+        auto put_powers = [&](const uint32_t (&r)[32]) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const float re = __uint_as_float(r[2 * j]), im = __uint_as_float(r[2 * j + 1]);
-                srow[j * 33] = re * re + im * im;
+            for (int j4 = 0; j4 < 4; ++j4) {
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float re = __uint_as_float(r[8 * j4 + 2 * j]), im = __uint_as_float(r[8 * j4 + 2 * j + 1]);
+                    v[j] = re * re + im * im;
+                }
+                *reinterpret_cast<float4*>(stg + 16 * lane + 4 * (j4 ^ ((lane >> 1) & 3))) =
+                    make_float4(v[0], v[1], v[2], v[3]);
             }
-            __syncwarp();
-            const int b16 = 16 * (c_begin + c);
-            const size_t row_base = static_cast<size_t>(un.shard) * jb.n_windows + jb.w0;
-            // two pairs per lane at a time (p and p + 32), their sums interleaved;
-            // a pair past the quadrant's reads the staging tile and is dropped
-            for (int pb = 0; pb < npairs; pb += 64) {
-                const int p0 = pb + lane, p1 = pb + 32 + lane;
-                const int j0 = p0 & 15, j1 = p1 & 15;
-                const int s0 = min(p0 >> 4, nwin_of(npairs) - 1), s1 = min(p1 >> 4, nwin_of(npairs) - 1);
-                const float* x0 = stg + j0 * 33 + s0 * sw;
-                const float* x1 = stg + j1 * 33 + s1 * sw;
+        };
+        auto staged = [&](int row) {
+            return *reinterpret_cast<const float2*>(stg + 16 * row + 4 * ((b_lane >> 2) ^ ((row >> 1) & 3)) +
+                                                    (b_lane & 2));
+        };
+        // Address arithmetic is what these sums must not repeat (with every row's
+        // offset formed, windows of 16 to 20 were 13 % slower), so the cases whose
+        // offsets are constants of the lane have their own loops.
+        int one_at[4];  // beam `lane` of a row 2 m (+ 1) modulo 8, for windows from row 0
+#pragma unroll
+        for (int m = 0; m < 4; ++m) one_at[m] = 4 * (((lane & 15) >> 2) ^ m) + (lane & 3);
+        // out: the first beam of this load in the quadrant's first window
+        auto sum_windows = [&](float* out, int beams_left, const TcJob& jb, int wq, int sw, int nwin) {
+            if (nwin == 1) {  // windows of 17 spectra or more: a lane per beam
+                float sum = 0.f;
+                int i = 0;
+#pragma unroll 1
+                for (; i + 8 <= sw; i += 8) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) sum += stg[16 * (i + k) + one_at[k >> 1]];
+                }
+#pragma unroll
+                for (int k = 0; k < 7; ++k) {
+                    if (i + k < sw) sum += stg[16 * (i + k) + one_at[k >> 1]];
+                }
+                if (lane < min(16, beams_left) && wq * sw < jb.n_time) out[lane] = sum;
+                return;
+            }
+            const size_t pitch = static_cast<size_t>(jb.n_freq) * jb.beam_stride;
+            for (int s = s_lane; s < nwin; s += 4) {
                 float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll 5
-                for (int i = 0; i < sw; ++i) {
-                    sum0 += x0[i];
-                    sum1 += x1[i];
+                auto add = [&](int row) {
+                    const float2 x = staged(row);
+                    sum0 += x.x;
+                    sum1 += x.y;
+                };
+                if (sw == 10) {  // the upchannelized cadence: all ten loads in flight
+#pragma unroll
+                    for (int i = 0; i < 10; ++i) add(10 * s + i);
+                } else if (sw == 16) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) add(16 * s + i);
+                } else {
+#pragma unroll 4
+                    for (int i = 0; i < sw; ++i) add(s * sw + i);
                 }
-                const int w0 = wq + s0, w1 = wq + s1;
-                if (p0 < npairs && w0 * sw < jb.n_time && b16 + j0 < jb.n_beams) {
-                    jb.integrated[((row_base + w0) * jb.n_freq + un.f) * jb.beam_stride + b16 + j0] = sum0;
-                }
-                if (p1 < npairs && w1 * sw < jb.n_time && b16 + j1 < jb.n_beams) {
-                    jb.integrated[((row_base + w1) * jb.n_freq + un.f) * jb.beam_stride + b16 + j1] = sum1;
+                if ((wq + s) * sw >= jb.n_time) continue;
+                float* dst = out + s * pitch + b_lane;
+                if (b_lane + 1 < beams_left && (jb.beam_stride & 1) == 0) {
+                    *reinterpret_cast<float2*>(dst) = make_float2(sum0, sum1);
+                } else {
+                    if (b_lane < beams_left) dst[0] = sum0;
+                    if (b_lane + 1 < beams_left) dst[1] = sum1;
                 }
             }
-            __syncwarp();
         };
         JobCursor<kServed> cur;
         if (u_begin < u_end) cur.init(p, u_begin);
@@ -811,41 +850,36 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             const Unit un = cur.at(unit_at(p, u));
             const TcJob& jb = cur.jb;
             const bool short_win = jb.spectra < 32;
-            const int sw = jb.spectra, nwin = short_win ? jb.rows_q / sw : 0, npairs = nwin * 16;
+            const int sw = jb.spectra, nwin = short_win ? jb.rows_q / sw : 0;
             for (int k = un.tile_begin; k < un.tile_end; ++k) {
                 if (!failed && !mbar_wait(&acc_full[acc_stage], acc_phase, kWaitNs)) { fail(128); failed = true; }
                 tc_fence_after();
                 const uint32_t taddr = tmem_base + ((32u * q4) << 16) + acc_stage * ACC_COLS + 32 * c_begin;
+                bool released = false;
                 if (short_win) {
                     const int sq = (4 * k + q4) * jb.rows_q;  // first spectrum of this quadrant
                     const int wq = (4 * k + q4) * nwin;         // its first window (rows_q = nwin * sw)
-                    if (!failed && sq < jb.n_time && kHalfLoads % 2 == 0) {
-                        // one load at a time: with two loads in flight beside the
-                        // staging sums, two loads per half spilled registers and
-                        // four ran 2-3 % slower (three stay faster paired)
+                    if (!failed && sq < jb.n_time) {
+                        const size_t row = static_cast<size_t>(un.shard) * jb.n_windows + jb.w0 + wq;
+                        float* out = jb.integrated + (row * jb.n_freq + un.f) * jb.beam_stride + 16 * c_begin;
+                        // One load at a time (the next one in flight beside the sums
+                        // was 8-15 % slower at three and four loads per half and
+                        // spilled at two); the MMAs get the accumulator back before
+                        // the last sums.
 #pragma unroll 1
                         for (int c = 0; c < c_count; ++c) {
-                            uint32_t r0[32];
-                            tmem_ld_32x32b_x32(taddr + 32 * c, r0);
+                            uint32_t r[32];
+                            tmem_ld_32x32b_x32(taddr + 32 * c, r);
                             tmem_ld_wait();
-                            short_windows(r0, c, jb, un, wq, sw, npairs);
+                            put_powers(r);
+                            const bool last = c + 1 == c_count;
+                            if (last) tc_fence_before();
+                            __syncwarp();
+                            if (last && lane == 0) mbar_arrive(&acc_empty[acc_stage]);
+                            sum_windows(out + 16 * c, jb.n_beams - 16 * (c_begin + c), jb, wq, sw, nwin);
+                            __syncwarp();
                         }
-                    } else if (!failed && sq < jb.n_time) {
-#pragma unroll
-                        for (int c = 0; c < kHalfLoads; c += 2) {
-                            uint32_t r0[32];
-                            if (c < c_count) tmem_ld_32x32b_x32(taddr + 32 * c, r0);
-                            if constexpr (kHalfLoads > 1) {
-                                uint32_t r1[32];
-                                if (c + 1 < c_count) tmem_ld_32x32b_x32(taddr + 32 * (c + 1), r1);
-                                tmem_ld_wait();
-                                if (c < c_count) short_windows(r0, c, jb, un, wq, sw, npairs);
-                                if (c + 1 < c_count) short_windows(r1, c + 1, jb, un, wq, sw, npairs);
-                            } else {
-                                tmem_ld_wait();
-                                if (c < c_count) short_windows(r0, c, jb, un, wq, sw, npairs);
-                            }
-                        }
+                        released = c_count > 0;
                     }
                 } else {
                     const int row0 = k * kTileM + 32 * q4;
@@ -871,9 +905,11 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                         cur_win = my_win;
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0 && !failed) mbar_arrive(&acc_empty[acc_stage]);
+                if (!released) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0 && !failed) mbar_arrive(&acc_empty[acc_stage]);
+                }
                 if (++acc_stage == 2) { acc_stage = 0; acc_phase ^= 1; }
 
                 const int tile_end_row = min((k + 1) * kTileM, jb.n_time);
@@ -919,8 +955,15 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                 // one decision for all epilogue warps, at the end of each unit (and
                 // every tile with fused quantization): stop together or go on
                 // together; a failed wait only makes the remaining tiles of the
-                // unit skip their work
-                if ((k + 1 == un.tile_end || fused) &&
+                // unit skip their work.  With short windows the warps share nothing
+                // (a unit is one tile there, so that would be a barrier per
+                // tile); each stops by itself.
+                if (short_win && !fused) {
+                    if (failed || *s_fail != 0) {
+                        stop = true;
+                        break;
+                    }
+                } else if ((k + 1 == un.tile_end || fused) &&
                     named_barrier_or(1, kEpiThreads, failed || *s_fail != 0)) {
                     stop = true;
                     break;
