@@ -375,10 +375,15 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
     // warps cover the 128 rows) and the MMAs read A from TMEM, which leaves
     // the shared memory to the weight images of up to 64 (32) beams.
     constexpr bool kTmemA = A >= 128;
-    constexpr int kXStages = A == 256 ? 1 : 2;
+    // Unpacking and MMAs hand over 128 antennas at a time (a stage is 128
+    // columns): with a whole 256-antenna row per stage only one fitted beside
+    // the accumulators and the two took turns (8192 spectra, 64 beams, windows
+    // of 320: 1.10 -> 0.95 ms).
+    constexpr int kXStages = A == 256 ? 3 : 2;
     constexpr int kHalvesA = A >= 128 ? A / 128 : 1;   // 128-byte halves of a raw row
+    constexpr uint32_t X_COLS = K / 2 / kHalvesA;      // TMEM columns of a voltage stage
     constexpr uint32_t A_COL0 = 2 * ACC_COLS;
-    static_assert(!kTmemA || A_COL0 + kXStages * (K / 2) <= 512, "TMEM holds two accumulators and the voltage");
+    static_assert(!kTmemA || A_COL0 + kXStages * X_COLS <= 512, "TMEM holds two accumulators and the voltage");
     constexpr uint32_t TMEM_COLS = kTmemA ? 512 : (2 * N <= 32) ? 32 : (2 * N <= 64) ? 64 : (2 * N <= 128) ? 128
                                    : (2 * N <= 256) ? 256 : 512;
     constexpr uint32_t IDESC = idesc_f16_f32(kTileM, N);
@@ -407,18 +412,18 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
     constexpr int kRawStages = static_cast<int>(S.raw_stages);
     uint64_t* raw_full = bars + 0;    // [kRawStages]
     uint64_t* raw_empty = bars + 4;   // [kRawStages]
-    uint64_t* x_full = bars + 8;      // [2]
-    uint64_t* x_empty = bars + 10;    // [2]
-    uint64_t* acc_full = bars + 12;   // [2]
-    uint64_t* acc_empty = bars + 14;  // [2]
-    uint64_t* w_full = bars + 16;     // [w_stages]
-    uint64_t* w_empty = bars + 18;    // [w_stages]
-    uint64_t* mma_done = bars + 20;
-    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 22);
-    volatile int* s_fail = reinterpret_cast<volatile int*>(bars + 23);
-    volatile int* s_quant = reinterpret_cast<volatile int*>(bars + 24);  // [8] windows to quantize
-    volatile int* s_meta = reinterpret_cast<volatile int*>(bars + 28);   // [2] their shard, channel group
-    static_assert(kRawStages <= kMaxRawStages && 29 * 8 <= 256, "barrier block");
+    uint64_t* x_full = bars + 8;      // [kXStages]
+    uint64_t* x_empty = bars + 11;    // [kXStages]
+    uint64_t* acc_full = bars + 14;   // [2]
+    uint64_t* acc_empty = bars + 16;  // [2]
+    uint64_t* w_full = bars + 18;     // [w_stages]
+    uint64_t* w_empty = bars + 20;    // [w_stages]
+    uint64_t* mma_done = bars + 22;
+    uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 23);
+    volatile int* s_fail = reinterpret_cast<volatile int*>(bars + 24);
+    volatile int* s_quant = reinterpret_cast<volatile int*>(bars + 25);  // [8] windows to quantize
+    volatile int* s_meta = reinterpret_cast<volatile int*>(bars + 29);   // [2] their shard, channel group
+    static_assert(kRawStages <= kMaxRawStages && kXStages <= 3 && 30 * 8 <= 256, "barrier block");
     // A list launch with an empty list (the checked form's common case) ends
     // before any set-up; every thread reads the same count.
     if (!kServed && p.unit_list != nullptr && *p.unit_count == 0) return;
@@ -436,9 +441,11 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             mbar_init(&raw_full[i], 1);
             mbar_init(&raw_empty[i], kUnpackWarps);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kXStages; ++i) {
             mbar_init(&x_full[i], kUnpackWarps);
             mbar_init(&x_empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], kEpiWarps);
         }
@@ -590,35 +597,42 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                 }
                 for (int k = un.tile_begin; k < un.tile_end; ++k) {
                     if (*s_fail) { stop = true; break; }
-                    if (!mbar_wait(&x_full[xs_stage], x_phase, kWaitNs)) { fail(8); stop = true; break; }
                     if (!mbar_wait(&acc_empty[acc_stage], acc_phase ^ 1, kWaitNs)) { fail(16); stop = true; break; }
-                    tc_fence_after();
                     const uint32_t d_tmem = tmem_base + acc_stage * ACC_COLS;
                     // descriptors once per tile; the start address field (bits 0-13,
                     // 16-byte units) then advances by plain adds (shared addresses stay
                     // below 2^18 bytes, so the field never carries)
-                    const uint64_t a0 = kTmemA ? 0 : smem_desc_sw128(smem_u32(xs + xs_stage * S.x_bytes));
-                    const uint32_t a_t = tmem_base + A_COL0 + xs_stage * (K / 2);  // voltage stage in TMEM
                     const uint64_t bh0 = smem_desc_sw128(w_hi_addr), bl0 = smem_desc_sw128(w_lo_addr);
+#pragma unroll 1
+                    for (int h = 0; h < kHalvesA; ++h) {
+                        if (!mbar_wait(&x_full[xs_stage], x_phase, kWaitNs)) { fail(8); stop = true; break; }
+                        tc_fence_after();
+                        const uint64_t a0 = kTmemA ? 0 : smem_desc_sw128(smem_u32(xs + xs_stage * S.x_bytes));
+                        const uint32_t a_t = tmem_base + A_COL0 + xs_stage * X_COLS;  // voltage stage in TMEM
+                        constexpr int kSteps = K / 16 / kHalvesA;
+                        const uint64_t b_half = h * ((kSteps / 4 * (N * 128)) >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < K / 16; ++kk) {
-                        const uint32_t kb = kk / 4, koff = (kk % 4) * 32;
-                        const uint64_t a = a0 + ((kb * (kTileM * 128) + koff) >> 4);
-                        const uint64_t bh = bh0 + ((kb * (N * 128) + koff) >> 4);
-                        const uint64_t bl = bl0 + ((kb * (N * 128) + koff) >> 4);
-                        if constexpr (kTmemA) {
-                            // 16 K values = 8 columns of the TMEM voltage stage
-                            mma_f16_ts(d_tmem, a_t + 8 * kk, bh, IDESC, kk > 0 ? 1u : 0u);
-                            mma_f16_ts(d_tmem, a_t + 8 * kk, bl, IDESC, 1u);
-                        } else {
-                            mma_f16_ss(d_tmem, a, bh, IDESC, kk > 0 ? 1u : 0u);
-                            mma_f16_ss(d_tmem, a, bl, IDESC, 1u);
+                        for (int kk = 0; kk < kSteps; ++kk) {
+                            const uint32_t kb = kk / 4, koff = (kk % 4) * 32;
+                            const uint64_t a = a0 + ((kb * (kTileM * 128) + koff) >> 4);
+                            const uint64_t bh = bh0 + b_half + ((kb * (N * 128) + koff) >> 4);
+                            const uint64_t bl = bl0 + b_half + ((kb * (N * 128) + koff) >> 4);
+                            const uint32_t accumulate = h > 0 || kk > 0 ? 1u : 0u;
+                            if constexpr (kTmemA) {
+                                // 16 K values = 8 columns of the TMEM voltage stage
+                                mma_f16_ts(d_tmem, a_t + 8 * kk, bh, IDESC, accumulate);
+                                mma_f16_ts(d_tmem, a_t + 8 * kk, bl, IDESC, 1u);
+                            } else {
+                                mma_f16_ss(d_tmem, a, bh, IDESC, accumulate);
+                                mma_f16_ss(d_tmem, a, bl, IDESC, 1u);
+                            }
                         }
+                        tc_commit(&x_empty[xs_stage]);
+                        if (++xs_stage == kXStages) { xs_stage = 0; x_phase ^= 1; }
                     }
-                    tc_commit(&x_empty[xs_stage]);
+                    if (stop) break;
                     tc_commit(&acc_full[acc_stage]);
                     if (k + 1 == un.tile_end && next_switches) tc_commit(&w_empty[ws]);
-                    if (++xs_stage == kXStages) { xs_stage = 0; x_phase ^= 1; }
                     if (++acc_stage == 2) { acc_stage = 0; acc_phase ^= 1; }
                 }
             }
@@ -650,40 +664,44 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             for (int k = un.tile_begin; k < un.tile_end; ++k) {
                 if (*s_fail) { stop = true; break; }
                 if (!mbar_wait(&raw_full[stage], phase, kWaitNs)) { fail(32); stop = true; break; }
-                if (!mbar_wait(&x_empty[xs_stage], x_phase ^ 1, kWaitNs)) { fail(64); stop = true; break; }
-                tc_fence_after();  // the MMAs that read this TMEM stage are complete
                 const uint8_t* row = raw + stage * S.raw_bytes + r * 128;
-                const uint32_t tbase = tmem_base + ((32u * q4) << 16) + A_COL0 + xs_stage * (K / 2);
+#pragma unroll 1
+                for (int half = 0; half < kHalvesA; ++half) {
+                    if (!mbar_wait(&x_empty[xs_stage], x_phase ^ 1, kWaitNs)) { fail(64); stop = true; break; }
+                    tc_fence_after();  // the MMAs that read this TMEM stage are complete
+                    const uint32_t tbase = tmem_base + ((32u * q4) << 16) + A_COL0 + xs_stage * X_COLS;
 #pragma unroll
-                for (int g4 = 0; g4 < A / 32; ++g4) {  // 32 columns: two 16-byte chunks of the row
-                    uint32_t col[32];
+                    for (int g4 = 0; g4 < 4; ++g4) {  // 32 columns: two 16-byte chunks of the 128-byte half
+                        uint32_t col[32];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int c = 2 * g4 + h;        // chunk c of the row: half c / 8, chunk c % 8 there
-                        uint4 w4 = *reinterpret_cast<const uint4*>(row + (c >> 3) * (kTileM * 128) +
-                                                                   (((c & 7) ^ (r & 7)) << 4));
-                        if (zero) w4 = make_uint4(0u, 0u, 0u, 0u);
-                        const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
+                        for (int h = 0; h < 2; ++h) {
+                            const int c = 2 * g4 + h;
+                            uint4 w4 = *reinterpret_cast<const uint4*>(row + half * (kTileM * 128) +
+                                                                       ((c ^ (r & 7)) << 4));
+                            if (zero) w4 = make_uint4(0u, 0u, 0u, 0u);
+                            const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const uint4 d4 = decode4(words[j]);
-                            col[16 * h + 4 * j + 0] = d4.x;
-                            col[16 * h + 4 * j + 1] = d4.y;
-                            col[16 * h + 4 * j + 2] = d4.z;
-                            col[16 * h + 4 * j + 3] = d4.w;
+                            for (int j = 0; j < 4; ++j) {
+                                const uint4 d4 = decode4(words[j]);
+                                col[16 * h + 4 * j + 0] = d4.x;
+                                col[16 * h + 4 * j + 1] = d4.y;
+                                col[16 * h + 4 * j + 2] = d4.z;
+                                col[16 * h + 4 * j + 3] = d4.w;
+                            }
                         }
+                        tmem_st_32x32b_x32(tbase + 32 * g4, col);
                     }
-                    tmem_st_32x32b_x32(tbase + 32 * g4, col);
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(&x_full[xs_stage]);
+                        if (half + 1 == kHalvesA) mbar_arrive(&raw_empty[stage]);
+                    }
+                    if (++xs_stage == kXStages) { xs_stage = 0; x_phase ^= 1; }
                 }
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(&raw_empty[stage]);
-                    mbar_arrive(&x_full[xs_stage]);
-                }
+                if (stop) break;
                 if (++stage == kRawStages) { stage = 0; phase ^= 1; }
-                if (++xs_stage == kXStages) { xs_stage = 0; x_phase ^= 1; }
             }
         }
       } else {
