@@ -1030,39 +1030,47 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
 // weight preparation: canonical complex64 -> split fp16 swizzled image
 // ------------------------------------------------------------------------
 // n_beams beams from b0 of canonical weights holding b_total beams per shard.
+// A thread forms one 16-byte K slot (4 antennas, in the decode's order) of a
+// beam's re and im rows, hi and lo: 32 bytes in, four 16-byte stores.  Bound
+// by its stores (64 antennas, 2 x 336 channels, 128 beams: 88 MB, 26 us;
+// 145 with a thread per 2-byte element).
 __global__ void prepare_split_kernel(const float2* __restrict__ w, uint8_t* __restrict__ out,
                                      int n_freq, int n_ant, int n_beams, int nb_pad, int n_shards, int b0,
                                      int b_total) {
-    const int K = 2 * n_ant, N = 2 * nb_pad;
-    const long long per_channel = static_cast<long long>(N) * K;
-    const long long total = per_channel * n_freq * n_shards;
+    const int K = 2 * n_ant, N = 2 * nb_pad, slots = n_ant / 4;
     const uint32_t w_bytes = (K / 64) * N * 128;
-    for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const long long ch = i / per_channel;  // shard * F + f
-        const int rem = static_cast<int>(i % per_channel);
-        const int n = rem / K, k = rem % K;
-        const int shard = static_cast<int>(ch / n_freq), f = static_cast<int>(ch % n_freq);
-        // inverse of the decode order: k -> (antenna, component)
-        const int q = k / 32, j = (k % 32) / 8, pslot = k % 8;
-        static constexpr int kAnt[8] = {0, 2, 0, 2, 1, 3, 1, 3};
-        static constexpr int kIm[8] = {0, 0, 1, 1, 0, 0, 1, 1};
-        const int a = 16 * q + 4 * j + kAnt[pslot];
-        const int comp = kIm[pslot];
-        const int b = n >> 1, out_im = n & 1;
-        float coef = 0.f;
-        if (b < n_beams) {
-            const float2 wv = w[((static_cast<size_t>(shard) * b_total + b0 + b) * n_freq + f) * n_ant + a];
-            // re out: x_re*wr - x_im*wi ; im out: x_re*wi + x_im*wr
-            coef = out_im ? (comp ? wv.x : wv.y) : (comp ? -wv.y : wv.x);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nb_pad * slots) return;
+    const int b = i / slots, s = i % slots;
+    for (int ch = blockIdx.y; ch < n_shards * n_freq; ch += gridDim.y) {
+        const int shard = ch / n_freq, f = ch % n_freq;
+        float2 wv[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            wv[a] = b < n_beams
+                        ? w[((static_cast<size_t>(shard) * b_total + b0 + b) * n_freq + f) * n_ant + 4 * s + a]
+                        : make_float2(0.f, 0.f);
         }
-        const __half hi = __float2half_rn(coef);
-        const __half lo = __float2half_rn(coef - __half2float(hi));
-        const int kb = k / 64, kk = k % 64;
-        const uint32_t off = kb * (N * 128) + n * 128 + ((((kk >> 3) ^ (n & 7))) << 4) + (kk & 7) * 2;
-        uint8_t* base = out + ch * 2 * w_bytes;
-        *reinterpret_cast<__half*>(base + off) = hi;
-        *reinterpret_cast<__half*>(base + w_bytes + off) = lo;
+        uint8_t* base = out + static_cast<size_t>(ch) * 2 * w_bytes + (s / 8) * (N * 128);
+#pragma unroll
+        for (int im = 0; im < 2; ++im) {
+            // re out: x_re*wr - x_im*wi ; im out: x_re*wi + x_im*wr, in the slot's order
+            // [re a0, re a2, im a0, im a2, re a1, re a3, im a1, im a3]
+            alignas(16) __half2 hi[4], lo[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const float2 x = wv[h >> 1], y = wv[(h >> 1) + 2];
+                const bool of_im = (h & 1) != 0;
+                const float c0 = im ? (of_im ? x.x : x.y) : (of_im ? -x.y : x.x);
+                const float c1 = im ? (of_im ? y.x : y.y) : (of_im ? -y.y : y.x);
+                hi[h] = __halves2half2(__float2half_rn(c0), __float2half_rn(c1));
+                lo[h] = __halves2half2(__float2half_rn(c0 - __low2float(hi[h])), __float2half_rn(c1 - __high2float(hi[h])));
+            }
+            const int n = 2 * b + im;
+            uint8_t* dst = base + n * 128 + (((s % 8) ^ (n & 7)) << 4);
+            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(hi);
+            *reinterpret_cast<uint4*>(dst + w_bytes) = *reinterpret_cast<const uint4*>(lo);
+        }
     }
 }
 
@@ -1165,14 +1173,17 @@ uint64_t split_weight_bytes(const bf_dims& d, uint64_t n_shards, int nb_pad) {
 
 bf_status launch_prepare_split(cudaStream_t stream, const float* w, void* split, const bf_dims& d,
                                uint64_t n_shards, int nb_pad) {
+    if (n_shards * d.n_freq > 0x7fffffffull) return set_error(BF_ERR_OVERFLOW, "too many shards");
+    auto prepare_grid = [&](int nbp) {
+        return dim3(static_cast<unsigned>((nbp * d.n_ant / 4 + 255) / 256),
+                    static_cast<unsigned>(std::min<uint64_t>(n_shards * d.n_freq, 32768)));
+    };
     if (beam_groups(d.n_ant)) {
         if (nb_pad > 0) return set_error(BF_ERR_UNSUPPORTED, "served jobs use 32 or 64 antennas");
         uint8_t* out = static_cast<uint8_t*>(split);
         for (int g = 0; g < group_count(d); ++g) {
             const int nb = group_beams(d, g), nbp = padded_beams(nb);
-            const long long total = static_cast<long long>(n_shards) * d.n_freq * 2 * nbp * 2 * d.n_ant;
-            const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 32));
-            prepare_split_kernel<<<blocks, 256, 0, stream>>>(
+            prepare_split_kernel<<<prepare_grid(nbp), 256, 0, stream>>>(
                 reinterpret_cast<const float2*>(w), out, static_cast<int>(d.n_freq), static_cast<int>(d.n_ant), nb,
                 nbp, static_cast<int>(n_shards), g * group_size(d), static_cast<int>(d.n_beams));
             BF_RETURN_IF(cuda_status(cudaGetLastError(), "prepare_split_kernel launch"));
@@ -1181,13 +1192,10 @@ bf_status launch_prepare_split(cudaStream_t stream, const float* w, void* split,
         return BF_OK;
     }
     const int nbp = nb_pad > 0 ? nb_pad : padded_beams(d.n_beams);
-    const long long total = static_cast<long long>(n_shards) * d.n_freq * 2 * nbp * 2 * d.n_ant;
-    const int blocks = static_cast<int>(std::min<long long>((total + 255) / 256, 148LL * 32));
-    prepare_split_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const float2*>(w),
-                                                     static_cast<uint8_t*>(split), static_cast<int>(d.n_freq),
-                                                     static_cast<int>(d.n_ant), static_cast<int>(d.n_beams),
-                                                     nbp, static_cast<int>(n_shards), 0,
-                                                     static_cast<int>(d.n_beams));
+    prepare_split_kernel<<<prepare_grid(nbp), 256, 0, stream>>>(
+        reinterpret_cast<const float2*>(w), static_cast<uint8_t*>(split), static_cast<int>(d.n_freq),
+        static_cast<int>(d.n_ant), static_cast<int>(d.n_beams), nbp, static_cast<int>(n_shards), 0,
+        static_cast<int>(d.n_beams));
     return cuda_status(cudaGetLastError(), "prepare_split_kernel launch");
 }
 
