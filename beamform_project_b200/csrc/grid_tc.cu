@@ -239,6 +239,26 @@ struct JobCursor {
         r.key = (j << 16) + r.shard * jb.n_freq + r.f;
         return r;
     }
+
+    // Entry i of the CTA's range [.., i_end) and, except in a list launch, the
+    // units of the same channel after it as one unit: n entries in all.  The
+    // roles then pay for finding their work once per channel instead of once
+    // per unit (a tile, with short windows): the MMA issuer spent 1000-1400
+    // clocks per tile outside its waits and MMAs.  64 antennas, 8000 spectra: 16
+    // beams in windows of 10 0.221 -> 0.158 ms, 64 in windows of 64 0.332 ->
+    // 0.252; 1024 spectra of 32 antennas, 16 beams 29.3 -> 24.6 us.
+    __device__ __forceinline__ Unit run(const TcParams& p, long long i, long long i_end, int& n) {
+        const long long u = unit_at(p, i);
+        Unit r = at(u);
+        n = 1;
+        if (kServed || p.unit_list == nullptr) {
+            n = static_cast<int>(min(static_cast<long long>(jb.groups_per_channel - d_g), i_end - i));
+            r.tile_end = min(r.tile_begin + n * jb.group_tiles, jb.tiles_per_channel);
+            d_g += n - 1;
+            last_u = u + n - 1;
+        }
+        return r;
+    }
 };
 
 // ---------------- fused quantization bookkeeping (epilogue thread 0) ----------
@@ -499,8 +519,9 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             JobCursor<kServed> cur;
             if (u_begin < u_end) cur.init(p, u_begin);
             cur.pair_parity = pair_parity;
-            for (long long u = u_begin; u < u_end && !stop; ++u) {
-                const Unit un = cur.at(unit_at(p, u));
+            int n = 0;
+            for (long long u = u_begin; u < u_end && !stop; u += n) {
+                const Unit un = cur.run(p, u, u_end, n);
                 const TcJob& jb = cur.jb;
                 if (un.key != prev_key) {
                     const uint32_t ws = w_loads % S.w_stages;
@@ -579,8 +600,9 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             JobCursor<kServed> cur;
             if (u_begin < u_end) cur.init(p, u_begin);
             cur.pair_parity = pair_parity;
-            for (long long u = u_begin; u < u_end && !stop; ++u) {
-                const Unit un = cur.at(unit_at(p, u));
+            int n = 0;
+            for (long long u = u_begin; u < u_end && !stop; u += n) {
+                const Unit un = cur.run(p, u, u_end, n);
                 if (un.key != prev_key) {
                     ws = w_switches % S.w_stages;
                     if (!mbar_wait(&w_full[ws], w_seen[ws] & 1, kWaitNs)) { fail(4); break; }
@@ -590,8 +612,10 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                     w_lo_addr = w_hi_addr + S.w_bytes;
                     prev_key = un.key;
                 }
+                // a run ends where its channel or the range does; a list may go on
+                // with another unit of the same channel
                 bool next_switches = true;
-                if (u + 1 < u_end) {
+                if (!kServed && p.unit_list != nullptr && u + 1 < u_end) {
                     JobCursor<kServed> ahead = cur;
                     next_switches = ahead.at(unit_at(p, u + 1)).key != un.key;
                 }
@@ -658,8 +682,9 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         JobCursor<kServed> cur;
         if (u_begin < u_end) cur.init(p, u_begin);
         cur.pair_parity = pair_parity;
-        for (long long u = u_begin; u < u_end && !stop; ++u) {
-            const Unit un = cur.at(unit_at(p, u));
+        int n = 0;
+        for (long long u = u_begin; u < u_end && !stop; u += n) {
+            const Unit un = cur.run(p, u, u_end, n);
             const bool zero = (r & 31) >= cur.jb.rows_q;  // spare quadrant rows of short windows
             for (int k = un.tile_begin; k < un.tile_end; ++k) {
                 if (*s_fail) { stop = true; break; }
@@ -714,8 +739,9 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         JobCursor<kServed> cur;
         if (u_begin < u_end) cur.init(p, u_begin);
         cur.pair_parity = pair_parity;
-        for (long long u = u_begin; u < u_end && !stop; ++u) {
-            const Unit un = cur.at(unit_at(p, u));
+        int n = 0;
+        for (long long u = u_begin; u < u_end && !stop; u += n) {
+            const Unit un = cur.run(p, u, u_end, n);
             const int R = cur.jb.rows_q;
             for (int k = un.tile_begin; k < un.tile_end; ++k) {
                 if (*s_fail) { stop = true; break; }
@@ -788,10 +814,10 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         // MMAs read 196 KB of operands and the powers cross it twice (128 KB),
         // 2900 clocks of its port against 2180 of MMAs, and two epilogue warps
         // per scheduler hide little of its latency (4200 clocks per tile, timed
-        // in the kernel).  Measured there, 8000 spectra in windows of 10: 0.457
-        // ms (0.481 with 4-byte stores and loads, addresses formed per sum and a
-        // barrier per tile), of 30 0.547 (0.625); 64 beams in windows of 10 0.300
-        // (0.342).
+        // in the kernel).  Measured there, 8000 spectra in windows of 10: 0.424
+        // ms (0.480 with 4-byte stores and loads, addresses formed per sum, and a
+        // barrier and a search for the next unit per tile); 64 beams in windows
+        // of 10 0.267 (0.343), of 24 0.408 (0.514).
         const int s_lane = lane >> 3, b_lane = 2 * (lane & 7);  // window, beams of this lane's sums
         auto put_powers = [&](const uint32_t (&r)[32]) {
 #pragma unroll
@@ -864,8 +890,9 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         JobCursor<kServed> cur;
         if (u_begin < u_end) cur.init(p, u_begin);
         cur.pair_parity = pair_parity;
-        for (long long u = u_begin; u < u_end && !stop; ++u) {
-            const Unit un = cur.at(unit_at(p, u));
+        int n = 0;
+        for (long long u = u_begin; u < u_end && !stop; u += n) {
+            const Unit un = cur.run(p, u, u_end, n);
             const TcJob& jb = cur.jb;
             const bool short_win = jb.spectra < 32;
             const int sw = jb.spectra, nwin = short_win ? jb.rows_q / sw : 0;
