@@ -72,8 +72,12 @@ __device__ __forceinline__ int find_job(const long long* begins, int stride_ll, 
 // a real-row column is the negated word).  Rows are XOR-swizzled so that the
 // 32 lanes of a fragment load hit 32 banks.
 // kShort (windows of at most 16 spectra: one row block) reads the fragments
-// where the MMAs use them instead of holding all four tiles in registers,
-// which leaves room for twice the resident CTAs.
+// where the MMAs use them instead of holding them in registers, which leaves
+// room for twice the resident CTAs.  Longer windows take the integer form of
+// tracker_common.cuh instead of fp16 parts, an m16n8k32 tile per source, with
+// the eight sources' digit fragments in registers; the plain tracker needs
+// that form, and here it costs what the fp16 form did (a mix of eight jobs,
+// three of them such trackers: 2.67 and 2.63 ms).
 // For one source the arithmetic (weights, fragments, MMA chain, hi + lo
 // combination, window sum order) is that of tracker_stream_kernel, so
 // results agree bit for bit (split(-x) is -split(x) except for the sign of a
@@ -111,7 +115,8 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
     using Frag = TrackerFrag<A>;
     constexpr int kWarpWords = 8 * 4 * Frag::kRowWords;  // 8 sources x 4 parts
     __shared__ double s_delay[2][8][A];  // by unit parity
-    __shared__ __align__(16) uint32_t s_frag[8][kWarpWords];
+    // fp16 part rows, or (long windows) the digit rows of four sources at a time
+    __shared__ __align__(16) uint32_t s_frag[8][kShort ? kWarpWords : kDigitRows * A];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
     const TrJob* jobs = reinterpret_cast<const TrJob*>(table + 1);
@@ -204,7 +209,7 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
             s_delay[db][sl][a] = steering_delay(jb.pos, a, d.x, d.y, d.z);
         }
         __syncthreads();
-        if (fvalid) {
+        if (kShort && fvalid) {
             // lane owns antennas lane + 32 c (its 16-bit slot in every part row
             // fixed); sources go in pairs, each row's offset a constant
             const double k = jb.kw[f];
@@ -239,60 +244,95 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         }
         __syncwarp();
 
-        // B fragments of the long form: column g of tile nt is (re, im) x
-        // (hi, lo) of source 8 sg + 2 nt + (g >> 2).
-        uint32_t bfrag[kShort ? 1 : 4][NW][2][2];
+        // Digit fragments of the long form: column g of source sl's tile.
+        uint32_t bfrag[kShort ? 1 : 8][NW][2];
         if constexpr (!kShort) {
+            const double k = fvalid ? jb.kw[f] : 0.0;
+            uint8_t* rows = reinterpret_cast<uint8_t*>(frag);
+            constexpr int kPairs = A / 2, kAtOnce = 32 / kPairs;  // sources formed by a warp at once
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
+            for (int s0 = 0; s0 < 8; s0 += 4) {
+                if (s0 < n_here) {
+                    __syncwarp();  // the last four sources' rows are read
+#pragma unroll 1
+                    for (int e = 0; e < 4; e += kAtOnce) {
+                        const int sl = s0 + e + lane / kPairs, pair = lane % kPairs;
+                        if (sl < n_here) {
+                            store_digits<A>(rows + (sl - s0) * kDigitRows * A, pair,
+                                            steering_from_delay(k, s_delay[db][sl][2 * pair]),
+                                            steering_from_delay(k, s_delay[db][sl][2 * pair + 1]));
+                        }
+                    }
+                    __syncwarp();
 #pragma unroll
-                for (int jj = 0; jj < NW; ++jj) {
-                    frag_load(nt, jj, bfrag[nt][jj][0][0], bfrag[nt][jj][0][1], bfrag[nt][jj][1][0],
-                              bfrag[nt][jj][1][1]);
+                    for (int e = 0; e < 4; ++e) {
+                        if (s0 + e < n_here) load_digit_frags<A>(rows + e * kDigitRows * A, g, q, bfrag[s0 + e]);
+                    }
                 }
             }
         }
 
-        float pw[4] = {0.f, 0.f, 0.f, 0.f};
+        float pw[kShort ? 4 : 8];
+#pragma unroll
+        for (int i = 0; i < (kShort ? 4 : 8); ++i) pw[i] = 0.f;
         for (int tb = t_begin; tb < t_end; tb += 16) {
             uint32_t ng[NW], ng8[NW];
             if constexpr (!kShort) load_rows(tb + 16, ng, ng8);
-            float d[4][4];
+            if constexpr (kShort) {
+                float d[4][4];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
+                for (int nt = 0; nt < 4; ++nt) d[nt][0] = d[nt][1] = d[nt][2] = d[nt][3] = 0.f;
 #pragma unroll
-            for (int jj = 0; jj < NW; ++jj) {
-                uint32_t re02g, im02g, re13g, im13g, re02h, im02h, re13h, im13h;
-                decode_word(wg[jj], re02g, im02g, re13g, im13g);
-                decode_word(wg8[jj], re02h, im02h, re13h, im13h);
+                for (int jj = 0; jj < NW; ++jj) {
+                    uint32_t re02g, im02g, re13g, im13g, re02h, im02h, re13h, im13h;
+                    decode_word(wg[jj], re02g, im02g, re13g, im13g);
+                    decode_word(wg8[jj], re02h, im02h, re13h, im13h);
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    if (nt < n_tiles) {
-                        if constexpr (kShort) {
+                    for (int nt = 0; nt < 4; ++nt) {
+                        if (nt < n_tiles) {
                             uint32_t b0r, b0i, b1r, b1i;
                             frag_load(nt, jj, b0r, b0i, b1r, b1i);
                             mma_16816(d[nt], re02g, re02h, im02g, im02h, b0r, b0i);
                             mma_16816(d[nt], re13g, re13h, im13g, im13h, b1r, b1i);
-                        } else {
-                            mma_16816(d[nt], re02g, re02h, im02g, im02h, bfrag[nt][jj][0][0], bfrag[nt][jj][0][1]);
-                            mma_16816(d[nt], re13g, re13h, im13g, im13h, bfrag[nt][jj][1][0], bfrag[nt][jj][1][1]);
                         }
                     }
                 }
-            }
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                if (nt < n_tiles) {
-                    // q == 0 / 2 hold (re_hi, im_hi) of the tile's first / second
-                    // source, q == 1 / 3 the lo parts, for rows g and g + 8
-                    float p[4];
+                for (int nt = 0; nt < 4; ++nt) {
+                    if (nt < n_tiles) {
+                        // q == 0 / 2 hold (re_hi, im_hi) of the tile's first / second
+                        // source, q == 1 / 3 the lo parts, for rows g and g + 8
+                        float p[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) p[i] = __shfl_xor_sync(0xffffffffu, d[nt][i], 1);
-                    const float re_g = d[nt][0] + p[0], im_g = d[nt][1] + p[1];
-                    const float re_h = d[nt][2] + p[2], im_h = d[nt][3] + p[3];
-                    const float pow_g = re_g * re_g + im_g * im_g;
-                    const float pow_h = re_h * re_h + im_h * im_h;
-                    pw[nt] += pow_g + pow_h;
+                        for (int i = 0; i < 4; ++i) p[i] = __shfl_xor_sync(0xffffffffu, d[nt][i], 1);
+                        const float re_g = d[nt][0] + p[0], im_g = d[nt][1] + p[1];
+                        const float re_h = d[nt][2] + p[2], im_h = d[nt][3] + p[3];
+                        const float pow_g = re_g * re_g + im_g * im_g;
+                        const float pow_h = re_h * re_h + im_h * im_h;
+                        pw[nt] += pow_g + pow_h;
+                    }
+                }
+            } else {
+                uint32_t re[2][NW], im[2][NW];
+#pragma unroll
+                for (int jj = 0; jj < NW; ++jj) {
+                    re[0][jj] = word_re16(wg[jj]);
+                    re[1][jj] = word_re16(wg8[jj]);
+                    im[0][jj] = word_im16(wg[jj]);
+                    im[1][jj] = word_im16(wg8[jj]);
+                }
+#pragma unroll
+                for (int sl = 0; sl < 8; ++sl) {
+                    if (sl < n_here) {
+                        int d[4] = {0, 0, 0, 0};
+#pragma unroll
+                        for (int jj = 0; jj < NW; ++jj) {
+                            mma_16832(d, re[0][jj], re[1][jj], im[0][jj], im[1][jj], bfrag[sl][jj][0], bfrag[sl][jj][1]);
+                        }
+                        float sq_g, sq_h;
+                        digit_squares<A>(d, q, sq_g, sq_h);
+                        pw[sl] = __fadd_rn(pw[sl], __fadd_rn(sq_g, sq_h));  // re^2 and im^2 apart until the window ends
+                    }
                 }
             }
             if constexpr (!kShort) {
@@ -304,14 +344,15 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
             }
         }
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            if (nt < n_tiles) {
-                float acc = pw[nt];
+        for (int i = 0; i < (kShort ? 4 : 8); ++i) {
+            if (i < (kShort ? n_tiles : n_here)) {
+                float acc = pw[i];
+                if constexpr (!kShort) acc += __shfl_xor_sync(0xffffffffu, acc, 2);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 4);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 8);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-                const int src = 8 * sg + 2 * nt + (q >> 1);
-                if (g == 0 && (q & 1) == 0 && fvalid && src < n_src) {
+                const int src = 8 * sg + (kShort ? 2 * i + (q >> 1) : i);
+                if (g == 0 && (kShort ? (q & 1) == 0 : q == 0) && fvalid && src < n_src) {
                     jb.integrated[(wglob * jb.n_freq + f) * n_src + src] = acc;
                 }
             }

@@ -116,5 +116,90 @@ __device__ __forceinline__ uint16_t split_part(float c, bool lo) {
     return __half_as_ushort(__float2half_rn(c - __half2float(h)));
 }
 
+// Integer form (windows above 16 spectra).  A weight w is the integer
+// q = rint(w 2^30) in four signed base-256 digits, exact for float weights of
+// at least 2^-7 and within 2^-31 below; voltages are 16 x the int4 values, one
+// mask per four components.  mma.m16n8k32 on int8 multiplies 16 spectra by 16
+// antennas (re in k 0-15, im in k 16-31) into the eight columns (re, im) x
+// (d3, d2, d1, d0), exactly.  Against the fp16 hi + lo form it halves the MMAs,
+// takes a third of the decode's instructions and rounds only when the digit
+// sums are put together; weights cost a third more to form, which a window of
+// one block does not earn back.
+
+// The digits of rint(w 2^30) as the bytes d0 .. d3, and those of its negative.
+struct Digits {
+    uint32_t pos, neg;
+};
+__device__ __forceinline__ Digits weight_digits(float w) {
+    const uint32_t q = static_cast<uint32_t>(__float2int_rn(__fmul_rn(w, 0x1p30f)));
+    return Digits{(q + 0x80808080u) ^ 0x80808080u, (0x80808080u - q) ^ 0x80808080u};
+}
+// Digit rows of a channel's weights in shared memory, one byte per antenna:
+// d3 .. d0 of Re w, of -Im w, of Im w.
+constexpr int kDigitRows = 12;
+// Antennas 2 pair and 2 pair + 1 of the rows.
+template <int A>
+__device__ __forceinline__ void store_digits(uint8_t* rows, int pair, float2 w0, float2 w1) {
+    const Digits x0 = weight_digits(w0.x), x1 = weight_digits(w1.x);
+    const Digits y0 = weight_digits(w0.y), y1 = weight_digits(w1.y);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(rows) + pair;
+#pragma unroll
+    for (int d = 0; d < 4; ++d) {
+        const uint32_t sel = 0x0073u - 0x11u * d;  // byte 3 - d of both
+        dst[d * (A / 2)] = static_cast<uint16_t>(__byte_perm(x0.pos, x1.pos, sel));
+        dst[(4 + d) * (A / 2)] = static_cast<uint16_t>(__byte_perm(y0.neg, y1.neg, sel));
+        dst[(8 + d) * (A / 2)] = static_cast<uint16_t>(__byte_perm(y0.pos, y1.pos, sel));
+    }
+}
+// B fragments (b0: re inputs, b1: im inputs) of column g of the MMAs over word
+// j of every lane quad's A / 4 antennas.
+template <int A>
+__device__ __forceinline__ void load_digit_frags(const uint8_t* rows, int g, int q, uint32_t (&b)[A / 16][2]) {
+    const uint8_t* r0 = rows + (g < 4 ? g : g + 4) * A + q * (A / 4);  // re: Re w; im: Im w
+    const uint8_t* r1 = rows + (g < 4 ? g + 4 : g - 4) * A + q * (A / 4);  // re: -Im w; im: Re w
+    if constexpr (A == 32) {
+        const uint2 x = *reinterpret_cast<const uint2*>(r0), y = *reinterpret_cast<const uint2*>(r1);
+        b[0][0] = x.x; b[1][0] = x.y; b[0][1] = y.x; b[1][1] = y.y;
+    } else {
+#pragma unroll
+        for (int j = 0; j < A / 16; j += 4) {
+            const uint4 x = *reinterpret_cast<const uint4*>(r0 + 4 * j), y = *reinterpret_cast<const uint4*>(r1 + 4 * j);
+            b[j][0] = x.x; b[j + 1][0] = x.y; b[j + 2][0] = x.z; b[j + 3][0] = x.w;
+            b[j][1] = y.x; b[j + 1][1] = y.y; b[j + 2][1] = y.z; b[j + 3][1] = y.w;
+        }
+    }
+}
+__device__ __forceinline__ void mma_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+        "{%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 16 x the real and imaginary parts of a word's four samples.
+__device__ __forceinline__ uint32_t word_re16(uint32_t w) { return (w << 4) & 0xF0F0F0F0u; }
+__device__ __forceinline__ uint32_t word_im16(uint32_t w) { return w & 0xF0F0F0F0u; }
+// The squared part of rows g and g + 8: re^2 in lanes q = 0 and 1, im^2 in 2
+// and 3.  Lane q even holds the sums of d3 and d2, odd those of d1 and d0; a
+// sum is at most 2 A 2^14 in magnitude, so 256 x one fits 32 bits up to 128
+// antennas.
+template <int A>
+__device__ __forceinline__ void digit_squares(const int (&d)[4], int q, float& sq_g, float& sq_h) {
+    const float scale = (q & 1) == 0 ? 0x1p-18f : 0x1p-34f;
+    float f[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        if constexpr (A <= 128) {
+            f[h] = __fmul_rn(__int2float_rn(d[2 * h] * 256 + d[2 * h + 1]), scale);
+        } else {
+            f[h] = __fmul_rn(__fmaf_rn(__int2float_rn(d[2 * h]), 256.0f, __int2float_rn(d[2 * h + 1])), scale);
+        }
+        f[h] = __fadd_rn(f[h], __shfl_xor_sync(0xffffffffu, f[h], 1));
+    }
+    sq_g = __fmul_rn(f[0], f[0]);
+    sq_h = __fmul_rn(f[1], f[1]);
+}
+
 }  // namespace trk
 }  // namespace bf

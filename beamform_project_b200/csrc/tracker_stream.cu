@@ -10,20 +10,24 @@
 // 12 ALU instructions per input byte, which would make the kernel ALU-bound,
 // so the MAC runs on the tensor pipe instead with the voltage fed straight
 // from registers:
-//   * Packed bytes are turned into fp16 pairs with two LOP3s (the nibble is
-//     placed in the mantissa of 1024.0 with its sign bit flipped) and one
-//     half2 subtract / fma -- int4 values are exact in fp16.
-//   * The weights are generated in registers once per window: FP64 delay
-//     and phase, reduced mod 2*pi in FP64, then float sin/cos, and split
-//     into an fp16 hi + lo pair (w = hi + lo to ~2^-22).
-//   * One mma.m16n8k16 (fp16 x fp16 -> fp32) multiplies 16 spectra x 8
-//     antennas by an 8-column weight matrix whose columns are (re, im) x
-//     (hi, lo) of the beam.  The hi and lo partial sums are added in fp32,
-//     then |.|^2.
+//   * Windows above 16 spectra use the integer form of tracker_common.cuh:
+//     voltages as int8 (16 x the int4 values, one mask per four components),
+//     each weight as four signed base-256 digits of rint(w 2^30), and one
+//     mma.m16n8k32 per 16 spectra x 16 antennas whose eight columns are
+//     (re, im) x the digits.  Everything before |.|^2 is exact but the last
+//     two roundings that put the digit sums together.
+//   * Windows of one block use fp16: packed bytes become fp16 pairs with two
+//     LOP3s (the nibble placed in the mantissa of 1024.0 with its sign bit
+//     flipped) and one half2 subtract / fma, weights an fp16 hi + lo pair, and
+//     mma.m16n8k16 multiplies 16 spectra x 8 antennas into (re, im) x (hi, lo),
+//     added in fp32.  There the digits would cost more to form than the
+//     shorter decode saves.
+//   * The weights come from FP64 delay and phase, reduced mod 2*pi in FP64,
+//     then float sin/cos.
 //   * Lanes (g, q) of the fragment map to spectra g, g+8 and to the q-th
 //     quarter of the antenna row, so each thread loads its A/4 contiguous
 //     bytes of two rows; the K order of the contraction is permuted to match
-//     the decode (only the weights need to follow it).
+//     (only the weights need to follow it).
 // A CTA of 8 warps takes 8 consecutive channels (512 contiguous bytes per
 // spectrum at 64 antennas), a warp one channel, in blocks of 16 spectra.  The
 // FP64 delays of the CTA's windows are formed once and each weight once per
@@ -37,13 +41,14 @@
 //     loads run ahead over the window ends without registers or barriers.
 // Per-spectrum powers are staged four blocks at a time so that each
 // spectrum's 8 channels are written as one 32-byte sector.
-// What bounds it: instruction issue with HBM close behind for long windows;
-// for windows of 10 spectra the weights' arithmetic and the six empty rows of
-// each block.
-// Measured at 64 antennas: 15360 spectra in windows of 10 with both outputs
-// 0.252 ms (0.819 ms with weights formed per fragment and one window per
-// CTA), 32000 in windows of 320 0.166 ms (0.190), 131072 in windows of 1024
-// 0.637 ms = 4.4 TB/s (0.666).
+// What bounds it: HBM for long windows (131072 spectra in windows of 1024,
+// 64 antennas: 0.471 ms = 6.0 TB/s; in the fp16 form issue, 0.637 ms); for
+// windows of 10 spectra the weights' arithmetic and the six empty rows of
+// each block (15360 spectra, both outputs, 0.252 ms; 0.819 with weights formed
+// per fragment and one window per CTA).  Other windows at 64 antennas: 32000
+// spectra in windows of 320 0.126 ms (0.189 at first), 8000 in windows of 32
+// 0.050 (0.147).  Against 64 bits the window sums of the integer form are off
+// by 4-6e-8, those of the fp16 form by 5e-8 (32 antennas) to 4e-7 (256).
 #include "bf_internal.cuh"
 #include "tracker_common.cuh"
 
@@ -60,14 +65,22 @@ constexpr int kChannelsPerCta = 8;
 constexpr int kMaxRun = 16;         // windows per CTA
 constexpr int kRunSpectra = 160;    // a run is as many windows as fit, one at least
 constexpr int kWantedCtas = 4 * 4 * 148;
-// Longest window of the ring form: windows of 100 take 75 us in it and 77 us
-// in the long form (9999 spectra), windows of 320 179 and 166 us (32000).
+// Longest window of the ring form: in the fp16 form windows of 100 took 75 us
+// in it and 77 us in the long form (9999 spectra), windows of 320 179 and 166
+// us (32000).
 constexpr int kShortWindow = 64;
+// Longest window in the fp16 form (one block), here and in the served tracker;
+// longer ones take the integer form.
+constexpr int kHalfWindow = 16;
 constexpr int kStageBlocks = 4;     // blocks of per-spectrum powers between barriers
 
 // Blocks of 16 spectra in a warp's ring (1 KB each at 64 antennas).
 template <int A>
 __host__ __device__ constexpr int ring_depth() { return A == 32 ? 8 : A == 64 ? 4 : A == 128 ? 3 : 2; }
+
+// Bytes of a warp's weights: fp16 parts, or digit rows.
+template <int A, bool kInt8>
+__host__ __device__ constexpr int part_bytes() { return kInt8 ? kDigitRows * A : 8 * A; }
 
 template <int N>
 __device__ __forceinline__ void copy_async(uint32_t dst, const void* src, bool on) {
@@ -95,7 +108,7 @@ struct BlockCursor {
     }
 };
 
-template <int A, bool kRuns>
+template <int A, bool kRuns, bool kInt8>
 __global__ void __launch_bounds__(kChannelsPerCta * 32)
 tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ pos,
                       const double* __restrict__ kw, const float* __restrict__ dirs,
@@ -108,8 +121,8 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
     constexpr int kSlot = 16 * A;       // bytes of a block: [row half][copy][lane]
     extern __shared__ uint4 smem_raw[];
     uint8_t* ring_all = reinterpret_cast<uint8_t*>(smem_raw);               // [8 warps][kDepth][kSlot] (kRuns)
-    uint32_t* parts_all = reinterpret_cast<uint32_t*>(ring_all + (kRuns ? 8 * kDepth * kSlot : 0));  // [8][4][A / 2]
-    double* delays = reinterpret_cast<double*>(parts_all + 8 * 2 * A);      // [run][A]
+    uint8_t* parts_all = ring_all + (kRuns ? 8 * kDepth * kSlot : 0);       // [8][part_bytes]
+    double* delays = reinterpret_cast<double*>(parts_all + 8 * part_bytes<A, kInt8>());  // [run][A]
     float* stage = reinterpret_cast<float*>(delays + run * A);              // [2][kStageBlocks][16][8], with intensity
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -141,7 +154,7 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
     // the ring: loads of the run's blocks in order, kDepth - 1 ahead
     uint8_t* ring = ring_all + warp * kDepth * kSlot;
     const uint32_t ring_at = static_cast<uint32_t>(__cvta_generic_to_shared(ring)) + lane * kCopy;
-    BlockCursor ahead;
+    BlockCursor ahead{};
     int ahead_slot = 0;
     auto ring_load = [&]() {
         if (ahead.win < w_end) {
@@ -194,77 +207,117 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
     }
     __syncthreads();
 
-    // B fragments of a window: column g in (re_hi, im_hi, re_lo, im_lo, 0...).
+    // B fragments of a window: column g in (re_hi, im_hi, re_lo, im_lo, 0...),
+    // or in (re, im) x the four digits.
     const double k = fvalid ? kw[f] : 0.0;
-    uint32_t* parts = parts_all + warp * 2 * A;  // rows re_hi, im_hi, re_lo, im_lo of words (a, a + 2)
-    uint32_t bfrag[NW][2][2];
+    uint8_t* digits = parts_all + warp * part_bytes<A, kInt8>();
+    uint32_t* parts = reinterpret_cast<uint32_t*>(digits);  // rows re_hi, im_hi, re_lo, im_lo of words (a, a + 2)
+    uint32_t bfrag[NW][kInt8 ? 1 : 2][2];
     auto form_weights = [&](int w) {
         __syncwarp();  // the previous window's words are read
         const double* dl = delays + (w - w_begin) * A;
+        if constexpr (kInt8) {
 #pragma unroll
-        for (int i = 0; i < (A / 2 + 31) / 32; ++i) {
-            const int word = lane + 32 * i, a0 = 4 * (word >> 1) + (word & 1);
-            if (word < A / 2) {
-                const float2 w0 = steering_from_delay(k, dl[a0]), w1 = steering_from_delay(k, dl[a0 + 2]);
-#pragma unroll
-                for (int lo = 0; lo < 2; ++lo) {
-                    parts[lo * A + word] = split_part(w0.x, lo) | (static_cast<uint32_t>(split_part(w1.x, lo)) << 16);
-                    parts[lo * A + A / 2 + word] =
-                        split_part(w0.y, lo) | (static_cast<uint32_t>(split_part(w1.y, lo)) << 16);
+            for (int i = 0; i < (A / 2 + 31) / 32; ++i) {
+                const int pair = lane + 32 * i;
+                if (pair < A / 2) {
+                    store_digits<A>(digits, pair, steering_from_delay(k, dl[2 * pair]),
+                                    steering_from_delay(k, dl[2 * pair + 1]));
                 }
             }
-        }
-        __syncwarp();
-        // re: xr * wr - xi * wi; im: xr * wi + xi * wr (column g < 4; the rest are zero)
-        const bool is_im = (g & 1) != 0;
-        const uint32_t flip = is_im ? 0u : 0x80008000u;
-        const uint32_t* row_r = parts + ((g >> 1) & 1) * A + (is_im ? A / 2 : 0) + q * 2 * NW;
-        const uint32_t* row_i = parts + ((g >> 1) & 1) * A + (is_im ? 0 : A / 2) + q * 2 * NW;
+            __syncwarp();
+            uint32_t b[NW][2];
+            load_digit_frags<A>(digits, g, q, b);
 #pragma unroll
-        for (int j = 0; j < NW; j += 2) {
-            const uint4 r4 = *reinterpret_cast<const uint4*>(row_r + 2 * j);
-            const uint4 i4 = *reinterpret_cast<const uint4*>(row_i + 2 * j);
-            const uint32_t wr[4] = {r4.x, r4.y, r4.z, r4.w}, wi[4] = {i4.x, i4.y, i4.z, i4.w};
+            for (int j = 0; j < NW; ++j) {
+                bfrag[j][0][0] = b[j][0];
+                bfrag[j][0][1] = b[j][1];
+            }
+        } else {
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                bfrag[j + (s >> 1)][s & 1][0] = g < 4 ? wr[s] : 0u;
-                bfrag[j + (s >> 1)][s & 1][1] = g < 4 ? wi[s] ^ flip : 0u;
+            for (int i = 0; i < (A / 2 + 31) / 32; ++i) {
+                const int word = lane + 32 * i, a0 = 4 * (word >> 1) + (word & 1);
+                if (word < A / 2) {
+                    const float2 w0 = steering_from_delay(k, dl[a0]), w1 = steering_from_delay(k, dl[a0 + 2]);
+#pragma unroll
+                    for (int lo = 0; lo < 2; ++lo) {
+                        parts[lo * A + word] = split_part(w0.x, lo) | (static_cast<uint32_t>(split_part(w1.x, lo)) << 16);
+                        parts[lo * A + A / 2 + word] =
+                            split_part(w0.y, lo) | (static_cast<uint32_t>(split_part(w1.y, lo)) << 16);
+                    }
+                }
+            }
+            __syncwarp();
+            // re: xr * wr - xi * wi; im: xr * wi + xi * wr (column g < 4; the rest are zero)
+            const bool is_im = (g & 1) != 0;
+            const uint32_t flip = is_im ? 0u : 0x80008000u;
+            const uint32_t* row_r = parts + ((g >> 1) & 1) * A + (is_im ? A / 2 : 0) + q * 2 * NW;
+            const uint32_t* row_i = parts + ((g >> 1) & 1) * A + (is_im ? 0 : A / 2) + q * 2 * NW;
+#pragma unroll
+            for (int j = 0; j < NW; j += 2) {
+                const uint4 r4 = *reinterpret_cast<const uint4*>(row_r + 2 * j);
+                const uint4 i4 = *reinterpret_cast<const uint4*>(row_i + 2 * j);
+                const uint32_t wr[4] = {r4.x, r4.y, r4.z, r4.w}, wi[4] = {i4.x, i4.y, i4.z, i4.w};
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    bfrag[j + (s >> 1)][s & 1][0] = g < 4 ? wr[s] : 0u;
+                    bfrag[j + (s >> 1)][s & 1][1] = g < 4 ? wi[s] ^ flip : 0u;
+                }
             }
         }
     };
 
     float acc = 0.f;
+    auto stage_powers = [&](int staged, float pow_g, float pow_h) {
+        float* st = stage + staged * 16 * kChannelsPerCta + warp;
+        st[g * kChannelsPerCta] = pow_g;
+        st[(g + 8) * kChannelsPerCta] = pow_h;
+    };
     // One block: its spectra's powers into the window sum and the stage.
     auto process = [&](const uint32_t (&wd)[2][NW], int staged) {
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        if constexpr (kInt8) {
+            int d[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int j = 0; j < NW; ++j) {
-            uint32_t re02g, im02g, re13g, im13g, re02h, im02h, re13h, im13h;
-            decode_word(wd[0][j], re02g, im02g, re13g, im13g);
-            decode_word(wd[1][j], re02h, im02h, re13h, im13h);
-            mma_16816(d, re02g, re02h, im02g, im02h, bfrag[j][0][0], bfrag[j][0][1]);
-            mma_16816(d, re13g, re13h, im13g, im13h, bfrag[j][1][0], bfrag[j][1][1]);
-        }
-        // q == 0 holds (re_hi, im_hi), q == 1 holds (re_lo, im_lo) for rows g, g+8.
-        float p[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = __shfl_xor_sync(0xffffffffu, d[i], 1);
-        const float re_g = d[0] + p[0], im_g = d[1] + p[1];
-        const float re_h = d[2] + p[2], im_h = d[3] + p[3];
-        const float pow_g = re_g * re_g + im_g * im_g;
-        const float pow_h = re_h * re_h + im_h * im_h;
-        if (q == 0) {
-            acc += pow_g + pow_h;
+            for (int j = 0; j < NW; ++j) {
+                mma_16832(d, word_re16(wd[0][j]), word_re16(wd[1][j]), word_im16(wd[0][j]), word_im16(wd[1][j]),
+                          bfrag[j][0][0], bfrag[j][0][1]);
+            }
+            float sq_g, sq_h;
+            digit_squares<A>(d, q, sq_g, sq_h);
+            acc = __fadd_rn(acc, __fadd_rn(sq_g, sq_h));  // re^2 and im^2 apart until the window ends
             if (intensity != nullptr) {
-                float* st = stage + staged * 16 * kChannelsPerCta + warp;
-                st[g * kChannelsPerCta] = pow_g;
-                st[(g + 8) * kChannelsPerCta] = pow_h;
+                const float pow_g = __fadd_rn(sq_g, __shfl_xor_sync(0xffffffffu, sq_g, 2));
+                const float pow_h = __fadd_rn(sq_h, __shfl_xor_sync(0xffffffffu, sq_h, 2));
+                if (q == 0) stage_powers(staged, pow_g, pow_h);
+            }
+        } else {
+            float d[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < NW; ++j) {
+                uint32_t re02g, im02g, re13g, im13g, re02h, im02h, re13h, im13h;
+                decode_word(wd[0][j], re02g, im02g, re13g, im13g);
+                decode_word(wd[1][j], re02h, im02h, re13h, im13h);
+                mma_16816(d, re02g, re02h, im02g, im02h, bfrag[j][0][0], bfrag[j][0][1]);
+                mma_16816(d, re13g, re13h, im13g, im13h, bfrag[j][1][0], bfrag[j][1][1]);
+            }
+            // q == 0 holds (re_hi, im_hi), q == 1 holds (re_lo, im_lo) for rows g, g+8.
+            float p[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = __shfl_xor_sync(0xffffffffu, d[i], 1);
+            const float re_g = d[0] + p[0], im_g = d[1] + p[1];
+            const float re_h = d[2] + p[2], im_h = d[3] + p[3];
+            const float pow_g = re_g * re_g + im_g * im_g;
+            const float pow_h = re_h * re_h + im_h * im_h;
+            if (q == 0) {
+                acc += pow_g + pow_h;
+                if (intensity != nullptr) stage_powers(staged, pow_g, pow_h);
             }
         }
     };
     auto finish_window = [&](int w) {
         if (integrated == nullptr) return;
         float sum = acc;
+        if constexpr (kInt8) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         sum += __shfl_xor_sync(0xffffffffu, sum, 4);
         sum += __shfl_xor_sync(0xffffffffu, sum, 8);
         sum += __shfl_xor_sync(0xffffffffu, sum, 16);
@@ -346,10 +399,13 @@ bf_status launch_stream(cudaStream_t stream, const uint8_t* v, const float* pos,
     int run = std::max(1, std::min(kMaxRun, kRunSpectra / S));
     while (run > 1 && static_cast<long long>(channel_groups) * ((W + run - 1) / run) < kWantedCtas) run /= 2;
     const bool runs = S <= kShortWindow;
-    const size_t smem = (runs ? 8 * ring_depth<A>() * 16 * A : 0) + 8 * 2 * A * sizeof(uint32_t) +
-                        run * A * sizeof(double) +
+    const bool int8 = S > kHalfWindow;
+    const size_t smem = (runs ? 8 * ring_depth<A>() * 16 * A : 0) +
+                        8 * (int8 ? part_bytes<A, true>() : part_bytes<A, false>()) + run * A * sizeof(double) +
                         (intensity != nullptr ? 2 * kStageBlocks * 16 * kChannelsPerCta * sizeof(float) : 0);
-    auto kernel = runs ? tracker_stream_kernel<A, true> : tracker_stream_kernel<A, false>;
+    auto kernel = !runs  ? tracker_stream_kernel<A, false, true>
+                  : int8 ? tracker_stream_kernel<A, true, true>
+                         : tracker_stream_kernel<A, true, false>;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (err != cudaSuccess) return cuda_status(err, "tracker_stream_kernel smem attribute");
     const dim3 grid(static_cast<unsigned>((W + run - 1) / run), static_cast<unsigned>(channel_groups));
