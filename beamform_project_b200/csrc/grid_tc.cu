@@ -34,7 +34,7 @@
 //               running per-window sums (S >= 32) or a staging tile summed per
 //               (window, beam) inside the warp's lane quadrant (S < 32), and
 //               window totals over the four quadrants in a fixed order.
-// Pipelines: 2 raw stages (4 at 128 antennas), 2 fp16 stages, 2 TMEM
+// Pipelines: 2 raw stages (4 at 128 antennas), 2 fp16 stages (3 half rows at 256), 2 TMEM
 // accumulators, all mbarrier driven; every wait is bounded and records an
 // error code instead of hanging.
 //
@@ -389,8 +389,8 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
     constexpr int N = 2 * NB;
     constexpr uint32_t ACC_COLS = N;          // fp32 columns per accumulator
     // At 128 and 256 antennas the fp16 voltage tile (128 rows x K, 64 or
-    // 128 KB) lives in TMEM after the two accumulators, K / 2 columns per
-    // stage (two stages at 128 antennas, one at 256): the unpack warps write
+    // 128 KB) lives in TMEM after the two accumulators, 128 columns
+    // per stage of 128 antennas (two stages at 128 antennas, three at 256): the unpack warps write
     // it with tcgen05.st (a warp reaches one lane quadrant, so four unpack
     // warps cover the 128 rows) and the MMAs read A from TMEM, which leaves
     // the shared memory to the weight images of up to 64 (32) beams.
