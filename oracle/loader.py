@@ -177,8 +177,13 @@ _timing = False
 @contextlib.contextmanager
 def perf_build():
     """Route the ref_* wrappers to the performance build of the reference core
-    (the timed CPU baselines); parity checks use the default parity build."""
+    (the timed CPU baselines); parity checks use the default parity build.
+    Without a reference build there is nothing to route: the baselines then
+    time the oracle and say so."""
     global _timing
+    if not reference_available():
+        yield None
+        return
     prev = _timing
     _timing = True
     try:
