@@ -395,10 +395,11 @@ template <int A>
 bf_status launch_stream(cudaStream_t stream, const uint8_t* v, const float* pos, const double* k, const float* dirs,
                         float* intensity, float* integrated, int T, int F, int S, int W) {
     const int channel_groups = (F + kChannelsPerCta - 1) / kChannelsPerCta;
-    // windows per CTA: short windows share a CTA's ramp, as long as the launch fills the GPU
-    int run = std::max(1, std::min(kMaxRun, kRunSpectra / S));
-    while (run > 1 && static_cast<long long>(channel_groups) * ((W + run - 1) / run) < kWantedCtas) run /= 2;
     const bool runs = S <= kShortWindow;
+    // windows per CTA: short windows share a CTA's ramp, as long as the launch
+    // fills the GPU; the long form walks one window
+    int run = runs ? std::max(1, std::min(kMaxRun, kRunSpectra / S)) : 1;
+    while (run > 1 && static_cast<long long>(channel_groups) * ((W + run - 1) / run) < kWantedCtas) run /= 2;
     const bool int8 = S > kHalfWindow;
     const size_t smem = (runs ? 8 * ring_depth<A>() * 16 * A : 0) +
                         8 * (int8 ? part_bytes<A, true>() : part_bytes<A, false>()) + run * A * sizeof(double) +

@@ -98,3 +98,21 @@ def test_mode1_window_edges(cuda, orc, A, T, S, outputs):
         assert np.all(np.abs(inten.astype(np.float64) - ref) <= 1e-3 + 1e-5 * np.abs(ref))
     exp64 = orc.integrate(ref[..., None], T, F, 1, S)[..., 0].astype(np.float64)
     assert np.all(np.abs(integ - exp64) <= 1e-3 + 1e-5 * np.abs(exp64))
+
+
+@pytest.mark.parametrize("A,S,W", [(64, 17, 530), (32, 33, 243), (64, 64, 119), (32, 64, 119), (64, 65, 119),
+                                   (32, 65, 119), (64, 72, 119), (32, 80, 119), (64, 80, 119), (64, 81, 119)])
+@pytest.mark.parametrize("outputs", ["both", "integrated"])
+def test_mode1_runs_of_windows(cuda, orc, A, S, W, outputs):
+    """Launches with so many windows that a CTA keeps several of them where
+    the form allows it, around the length at which the one-window form
+    begins; the last window is partial and no window keeps the buffers' fill
+    value.  The tolerance is the file's."""
+    from beamform_project_b200 import api
+    T = (W - 1) * S + 7
+    pos, freq, dirs, v, ref = _case(orc, api, T, A, S, seed=S)
+    inten, integ = _run(cuda, api, 1, v, pos, freq, dirs, T, A, S, want_int=outputs == "both")
+    if inten is not None:
+        assert np.all(np.abs(inten.astype(np.float64) - ref) <= 1e-3 + 1e-5 * np.abs(ref))
+    exp64 = orc.integrate(ref[..., None], T, F, 1, S)[..., 0].astype(np.float64)
+    assert np.all(np.abs(integ - exp64) <= 1e-3 + 1e-5 * np.abs(exp64))
