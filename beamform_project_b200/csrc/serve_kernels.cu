@@ -115,6 +115,10 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
     using Frag = TrackerFrag<A>;
     constexpr int kWarpWords = 8 * 4 * Frag::kRowWords;  // 8 sources x 4 parts
     __shared__ double s_delay[2][8][A];  // by unit parity
+    // Long windows: the largest |delay| of a source's antennas, and per warp the
+    // sources whose weights have no digits (a phase that is not finite, or too
+    // large to have a value); their products are NaN.
+    __shared__ unsigned s_far[2][8][A / 32], s_no_digits[8];
     // fp16 part rows, or (long windows) the digit rows of four sources at a time
     __shared__ __align__(16) uint32_t s_frag[8][kShort ? kWarpWords : kDigitRows * A];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -206,7 +210,13 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         for (int i = threadIdx.x; i < n_here * A; i += blockDim.x) {
             const int sl = i / A, a = i % A;
             const float3 d = trajectory_direction(jb.traj + 4 * (8 * sg + sl), wglob * S);
-            s_delay[db][sl][a] = steering_delay(jb.pos, a, d.x, d.y, d.z);
+            const double delay = steering_delay(jb.pos, a, d.x, d.y, d.z);
+            s_delay[db][sl][a] = delay;
+            if constexpr (!kShort) {
+                // the largest of the warp's 32 antennas; a NaN is above every number
+                const unsigned far = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf(__double2float_ru(delay))));
+                if (lane == 0) s_far[db][sl][a / 32] = far;
+            }
         }
         __syncthreads();
         if (kShort && fvalid) {
@@ -248,6 +258,11 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         uint32_t bfrag[kShort ? 1 : 8][NW][2];
         if constexpr (!kShort) {
             const double k = fvalid ? jb.kw[f] : 0.0;
+            unsigned far = s_far[db][lane & 7][0];
+            if constexpr (A == 64) far = max(far, s_far[db][lane & 7][1]);
+            const bool phasors = fabsf(static_cast<float>(k)) * __uint_as_float(far) < 0x1p51f;
+            const unsigned no_digits = ~__ballot_sync(0xffffffffu, phasors);
+            if (lane == 0) s_no_digits[warp] = no_digits;
             uint8_t* rows = reinterpret_cast<uint8_t*>(frag);
             constexpr int kPairs = A / 2, kAtOnce = 32 / kPairs;  // sources formed by a warp at once
 #pragma unroll
@@ -330,7 +345,7 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
                             mma_16832(d, re[0][jj], re[1][jj], im[0][jj], im[1][jj], bfrag[sl][jj][0], bfrag[sl][jj][1]);
                         }
                         float sq_g, sq_h;
-                        digit_squares<A>(d, q, sq_g, sq_h);
+                        digit_squares<A>(d, digit_scale(q), sq_g, sq_h);
                         pw[sl] = __fadd_rn(pw[sl], __fadd_rn(sq_g, sq_h));  // re^2 and im^2 apart until the window ends
                     }
                 }
@@ -351,6 +366,7 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
                 acc += __shfl_xor_sync(0xffffffffu, acc, 4);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 8);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+                if (!kShort && ((s_no_digits[warp] >> i) & 1u) != 0) acc = NAN;
                 const int src = 8 * sg + (kShort ? 2 * i + (q >> 1) : i);
                 if (g == 0 && (kShort ? (q & 1) == 0 : q == 0) && fvalid && src < n_src) {
                     jb.integrated[(wglob * jb.n_freq + f) * n_src + src] = acc;

@@ -126,6 +126,24 @@ __device__ __forceinline__ uint16_t split_part(float c, bool lo) {
 // sums are put together; weights cost a third more to form, which a window of
 // one block does not earn back.
 
+// A weight has digits when it is finite and of the size a phasor can have; a
+// direction or wave number that is not finite gives one that has none.  Such a
+// (window, channel) must not come out as a finite power, as it does not in the
+// forms that keep weights as floats: its powers are NaN.  Weights are looked at
+// only where a delay or a wave number is out of the ordinary: inside both bounds
+// a phase is below 2^51 quadrants and its weight a phasor.
+__device__ __forceinline__ bool odd_delay(double delay) { return !(fabs(delay) < 0x1p40); }
+__device__ __forceinline__ bool odd_wave_number(double k) { return !(fabs(k) < 0x1p11); }
+__device__ __forceinline__ bool has_digits(float2 w) { return fabsf(w.x) < 1.5f && fabsf(w.y) < 1.5f; }
+// All of a window's weights, for the warp.
+template <int A>
+__device__ __forceinline__ bool weights_have_digits(double k, const double* delays, int lane) {
+    bool all = true;
+#pragma unroll 1
+    for (int a = lane; a < A; a += 32) all = all && has_digits(steering_from_delay(k, delays[a]));
+    return __all_sync(0xffffffffu, all);
+}
+
 // The digits of rint(w 2^30) as the bytes d0 .. d3, and those of its negative.
 struct Digits {
     uint32_t pos, neg;
@@ -180,13 +198,14 @@ __device__ __forceinline__ void mma_16832(int (&d)[4], uint32_t a0, uint32_t a1,
 // 16 x the real and imaginary parts of a word's four samples.
 __device__ __forceinline__ uint32_t word_re16(uint32_t w) { return (w << 4) & 0xF0F0F0F0u; }
 __device__ __forceinline__ uint32_t word_im16(uint32_t w) { return w & 0xF0F0F0F0u; }
+// What lane q's digit sums count: the lanes of d3 and d2 (q even), of d1 and d0.
+__device__ __forceinline__ float digit_scale(int q) { return (q & 1) == 0 ? 0x1p-18f : 0x1p-34f; }
 // The squared part of rows g and g + 8: re^2 in lanes q = 0 and 1, im^2 in 2
 // and 3.  Lane q even holds the sums of d3 and d2, odd those of d1 and d0; a
 // sum is at most 2 A 2^14 in magnitude, so 256 x one fits 32 bits up to 128
-// antennas.
+// antennas.  scale: digit_scale(q), or NaN for a window without digits.
 template <int A>
-__device__ __forceinline__ void digit_squares(const int (&d)[4], int q, float& sq_g, float& sq_h) {
-    const float scale = (q & 1) == 0 ? 0x1p-18f : 0x1p-34f;
+__device__ __forceinline__ void digit_squares(const int (&d)[4], float scale, float& sq_g, float& sq_h) {
     float f[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {

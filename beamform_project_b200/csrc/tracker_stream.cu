@@ -201,11 +201,13 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
         load_rows(cur.t, cur.end, wa);
         load_rows(cur.t + 16, cur.end, wb);
     }
+    bool odd = false;
     for (int i = threadIdx.x; i < (w_end - w_begin) * A; i += kChannelsPerCta * 32) {
         const float* d = dirs + 3 * (w_begin + i / A);
         delays[i] = steering_delay(pos, i % A, d[0], d[1], d[2]);
+        odd = odd || odd_delay(delays[i]);
     }
-    __syncthreads();
+    if constexpr (kInt8) odd = __syncthreads_or(odd) != 0; else __syncthreads();
 
     // B fragments of a window: column g in (re_hi, im_hi, re_lo, im_lo, 0...),
     // or in (re, im) x the four digits.
@@ -213,6 +215,8 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
     uint8_t* digits = parts_all + warp * part_bytes<A, kInt8>();
     uint32_t* parts = reinterpret_cast<uint32_t*>(digits);  // rows re_hi, im_hi, re_lo, im_lo of words (a, a + 2)
     uint32_t bfrag[NW][kInt8 ? 1 : 2][2];
+    const bool look = kInt8 && (odd || odd_wave_number(k));
+    float scale = digit_scale(q);  // of the digit sums; NaN for a window without digits
     auto form_weights = [&](int w) {
         __syncwarp();  // the previous window's words are read
         const double* dl = delays + (w - w_begin) * A;
@@ -225,6 +229,7 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
                                     steering_from_delay(k, dl[2 * pair + 1]));
                 }
             }
+            if (look) scale = weights_have_digits<A>(k, dl, lane) ? digit_scale(q) : NAN;
             __syncwarp();
             uint32_t b[NW][2];
             load_digit_frags<A>(digits, g, q, b);
@@ -283,7 +288,7 @@ tracker_stream_kernel(const uint8_t* __restrict__ v, const float* __restrict__ p
                           bfrag[j][0][0], bfrag[j][0][1]);
             }
             float sq_g, sq_h;
-            digit_squares<A>(d, q, sq_g, sq_h);
+            digit_squares<A>(d, scale, sq_g, sq_h);
             acc = __fadd_rn(acc, __fadd_rn(sq_g, sq_h));  // re^2 and im^2 apart until the window ends
             if (intensity != nullptr) {
                 const float pow_g = __fadd_rn(sq_g, __shfl_xor_sync(0xffffffffu, sq_g, 2));

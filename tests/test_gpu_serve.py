@@ -5,6 +5,8 @@ exactly), and the device weight generator matches the reference's
 generate_weights."""
 from __future__ import annotations
 
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -297,3 +299,24 @@ def test_windows_per_step_products(cuda):
             for a, b in zip(one[idx], many[idx]):
                 if a is not None:
                     assert np.array_equal(a, b), (k, idx)
+
+
+@pytest.mark.parametrize("A,S", [(32, 10), (64, 10), (32, 32), (64, 32), (32, 320), (64, 320)])
+def test_served_tracker_without_a_phase(cuda, A, S):
+    """An antenna so far out that its phase has no value gives NaN products
+    to the sources it delays, in both forms, and none to the sources at the
+    zenith, whose delays are zero."""
+    good = _tracker_job(A=A, ns=1, n_src=11, S=S)
+    tr = good.trajectories.copy()
+    zenith = np.array([0, 3, 6, 7, 9])
+    tr[zenith] = 0.0
+    tr[np.setdiff1d(np.arange(11), zenith), :2] += 0.01
+    good = dataclasses.replace(good, trajectories=tr)
+    pos = good.positions.copy()
+    pos[5, 0] = 1e30
+    with _server() as srv:
+        (a, _, _), (b, _, _) = _run(srv, [good, dataclasses.replace(good, positions=pos)])
+    assert np.isfinite(a).all()
+    nan = np.isnan(b).reshape(-1, 11)
+    assert not nan[:, zenith].any() and np.delete(nan, zenith, axis=1).all()
+    assert np.array_equal(b.reshape(-1, 11)[:, zenith], a.reshape(-1, 11)[:, zenith])

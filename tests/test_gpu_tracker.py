@@ -116,3 +116,35 @@ def test_mode1_runs_of_windows(cuda, orc, A, S, W, outputs):
         assert np.all(np.abs(inten.astype(np.float64) - ref) <= 1e-3 + 1e-5 * np.abs(ref))
     exp64 = orc.integrate(ref[..., None], T, F, 1, S)[..., 0].astype(np.float64)
     assert np.all(np.abs(integ - exp64) <= 1e-3 + 1e-5 * np.abs(exp64))
+
+
+@pytest.mark.parametrize("A", [32, 64, 256])
+@pytest.mark.parametrize("S", [10, 32, 320])
+def test_mode1_not_finite(cuda, orc, A, S):
+    """A window direction or wave number that is not finite gives NaN powers
+    in its window or channel, in every form of the streaming kernel as in the
+    reference order, and changes no other value."""
+    from beamform_project_b200 import api
+    torch = cuda
+    T = 3 * S + 5
+    pos, freq, dirs, v, _ = _case(orc, api, T, A, S, seed=S)
+    kw = np.asarray(api.wave_numbers(freq))
+    bad_dirs, bad_kw = dirs.copy(), kw.copy()
+    bad_dirs[1, 0], bad_dirs[3, 1] = np.nan, np.inf
+    bad_kw[11], bad_kw[330] = np.nan, np.inf
+
+    def run(mode, kw, dirs):
+        inten = torch.full((T * F,), -1.0, dtype=torch.float32, device="cuda")
+        integ = torch.full((4 * F,), -1.0, dtype=torch.float32, device="cuda")
+        api.tracker(None, mode, _dev(torch, v), _dev(torch, pos), _dev(torch, kw), _dev(torch, dirs), inten, integ,
+                    api.Dimensions(T, F, A, 1), S)
+        return inten.cpu().numpy().reshape(T, F), integ.cpu().numpy().reshape(4, F)
+
+    good, bad, order = run(1, kw, dirs), run(1, bad_kw, bad_dirs), run(0, bad_kw, bad_dirs)
+    win = np.zeros((4, F), bool)
+    win[[1, 3]] = True
+    win[:, [11, 330]] = True
+    expect = win[np.arange(T) // S], win
+    for g, b, o, e in zip(good, bad, order, expect):
+        assert np.array_equal(np.isnan(b), e) and np.array_equal(np.isnan(o), e)
+        assert np.array_equal(b[~e], g[~e])
