@@ -172,6 +172,10 @@ doa_search_kernel(TrackParams p, int b, SearchState* __restrict st, float* __res
     const int tid = threadIdx.x, group = static_cast<int>(cluster.block_rank());
     const int n_groups = static_cast<int>(gridDim.y);
     const int f0 = group * kChanGroup, nf = min(kChanGroup, p.n_freq - f0);
+    // A CTA's shared memory may be written from another one only once it is
+    // known to run: every CTA says so here and waits for the others before the
+    // first remote write, with the copies and the coarse sums in between.
+    cluster.barrier_arrive();
     // Up to the wait for the window before, a CTA touches only what the fold
     // wrote and the caller's arrays.
     const Cd* X0 = (p.capon ? p.Q : p.S) + (static_cast<size_t>(b) * p.n_freq + f0) * M * M;
@@ -264,6 +268,7 @@ doa_search_kernel(TrackParams p, int b, SearchState* __restrict st, float* __res
     const int i0 = blockIdx.x * kCoarseTile, np = min(kCoarseTile, n_points - i0);
     {
         const double s = point_sum(np, [&](int i) { return coarse_point(i0 + i, c0_l, c0_m, q.G, q.fov_l, q.fov_m); });
+        cluster.barrier_wait();
         if (tid < np) *cluster.map_shared_rank(&part[0][group][tid], 0) = s;
     }
     cluster.sync();
