@@ -52,6 +52,7 @@
 
 #include <climits>
 #include <mutex>
+#include <type_traits>
 
 namespace bf {
 
@@ -155,6 +156,17 @@ __device__ __forceinline__ float beam_pair_sum(const uint32_t (&r)[32], int lane
         v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
     }
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+__device__ __forceinline__ float ld_shared_f(uint32_t at) {
+    float x;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(at) : "memory");
+    return x;
+}
+__device__ __forceinline__ float2 ld_shared_f2(uint32_t at) {
+    float2 x;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x.x), "=f"(x.y) : "r"(at) : "memory");
+    return x;
 }
 
 struct Unit {
@@ -813,12 +825,14 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
         // What bounds it: shared memory.  At 64 antennas and 128 beams a tile's
         // MMAs read 196 KB of operands and the powers cross it twice (128 KB),
         // 2900 clocks of its port against 2180 of MMAs, and two epilogue warps
-        // per scheduler hide little of its latency (4200 clocks per tile, timed
-        // in the kernel).  Measured there, 8000 spectra in windows of 10: 0.424
-        // ms (0.480 with 4-byte stores and loads, addresses formed per sum, and a
-        // barrier and a search for the next unit per tile); 64 beams in windows
-        // of 10 0.267 (0.343), of 24 0.408 (0.514).
-        const int s_lane = lane >> 3, b_lane = 2 * (lane & 7);  // window, beams of this lane's sums
+        // per scheduler hide little of its latency (4200 clocks per tile before
+        // the addresses below, timed in the kernel).  Measured there, 8000
+        // spectra, with every length's addresses constant (with those of 10, 16
+        // and above 16 only; with 4-byte loads, addresses formed per sum, and a
+        // barrier and a search for the next unit per tile): windows of 1 0.594 ms
+        // (0.895; 1.296), of 7 0.395 (0.491; 0.527), of 10 0.390 (0.428; 0.486),
+        // of 15 0.397 (0.522; 0.504), of 16 0.382 (0.420; 0.491), of 24 0.537
+        // (0.621; 0.792); 48 beams in windows of 9 0.263 (0.308; 0.385).
         auto put_powers = [&](const uint32_t (&r)[32]) {
 #pragma unroll
             for (int j4 = 0; j4 < 4; ++j4) {
@@ -832,58 +846,69 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                     make_float4(v[0], v[1], v[2], v[3]);
             }
         };
-        auto staged = [&](int row) {
-            return *reinterpret_cast<const float2*>(stg + 16 * row + 4 * ((b_lane >> 2) ^ ((row >> 1) & 3)) +
-                                                    (b_lane & 2));
-        };
-        // Address arithmetic is what these sums must not repeat (with every row's
-        // offset formed, windows of 16 to 20 were 13 % slower), so the cases whose
-        // offsets are constants of the lane have their own loops.
-        int one_at[4];  // beam `lane` of a row 2 m (+ 1) modulo 8, for windows from row 0
+        // Address arithmetic is what these sums must not repeat.  Rows eight apart
+        // lie alike, so a lane's eight addresses stand for a whole run and a
+        // sum is loads at constant distances from them, for every length:
+        // up to 16 spectra by two beams of a window (set below), above by one beam
+        // of the quadrant's only window.
+        uint32_t row_at[8];
+        const int s_lane = lane >> 3, b_lane = 2 * (lane & 7);  // window, beams of this lane's sums
+        auto set_rows = [&](int sw) {
+            const uint32_t base = smem_u32(stg);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) one_at[m] = 4 * (((lane & 15) >> 2) ^ m) + (lane & 3);
-        // out: the first beam of this load in the quadrant's first window
-        auto sum_windows = [&](float* out, int beams_left, const TcJob& jb, int wq, int sw, int nwin) {
-            if (nwin == 1) {  // windows of 17 spectra or more: a lane per beam
-                float sum = 0.f;
-                int i = 0;
-#pragma unroll 1
-                for (; i + 8 <= sw; i += 8) {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) sum += stg[16 * (i + k) + one_at[k >> 1]];
-                }
-#pragma unroll
-                for (int k = 0; k < 7; ++k) {
-                    if (i + k < sw) sum += stg[16 * (i + k) + one_at[k >> 1]];
-                }
-                if (lane < min(16, beams_left) && wq * sw < jb.n_time) out[lane] = sum;
-                return;
+            for (int k = 0; k < 8; ++k) {
+                const int row = sw <= 16 ? sw * s_lane + k : k, b = sw <= 16 ? b_lane : lane & 15;
+                row_at[k] = base + 4u * (16 * row + 4 * ((b >> 2) ^ ((row >> 1) & 3)) + (b & 3));
             }
+        };
+        // out: the first beam of this load in the quadrant's first window
+        auto sum_windows = [&](auto length, float* out, int beams_left, const TcJob& jb, int wq) {
+            constexpr int SW = decltype(length)::value, kWindows = 32 / SW;
             const size_t pitch = static_cast<size_t>(jb.n_freq) * jb.beam_stride;
-            for (int s = s_lane; s < nwin; s += 4) {
+#pragma unroll
+            for (int s0 = 0; s0 < kWindows; s0 += 4) {
+                const int s = s0 + s_lane;
+                if (s >= kWindows) break;
                 float sum0 = 0.f, sum1 = 0.f;
-                auto add = [&](int row) {
-                    const float2 x = staged(row);
+#pragma unroll
+                for (int i = 0; i < SW; ++i) {
+                    // row SW s0 + i from the lane's first one; its place depends on it modulo 8
+                    const float2 x = ld_shared_f2(row_at[(SW * s0 + i) & 7] + 64u * ((SW * s0 + i) & ~7));
                     sum0 += x.x;
                     sum1 += x.y;
-                };
-                if (sw == 10) {  // the upchannelized cadence: all ten loads in flight
-#pragma unroll
-                    for (int i = 0; i < 10; ++i) add(10 * s + i);
-                } else if (sw == 16) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) add(16 * s + i);
-                } else {
-#pragma unroll 4
-                    for (int i = 0; i < sw; ++i) add(s * sw + i);
                 }
-                if ((wq + s) * sw >= jb.n_time) continue;
+                if ((wq + s) * SW >= jb.n_time) continue;
                 float* dst = out + s * pitch + b_lane;
                 if (b_lane + 1 < beams_left && (jb.beam_stride & 1) == 0) {
                     *reinterpret_cast<float2*>(dst) = make_float2(sum0, sum1);
                 } else {
                     if (b_lane < beams_left) dst[0] = sum0;
                     if (b_lane + 1 < beams_left) dst[1] = sum1;
+                }
+            }
+        };
+        auto sum_short = [&](float* out, int beams_left, const TcJob& jb, int wq, int sw) {
+            switch (sw) {
+#define BF_LENGTH(n) \
+    case n: sum_windows(std::integral_constant<int, n>{}, out, beams_left, jb, wq); break;
+                BF_LENGTH(1) BF_LENGTH(2) BF_LENGTH(3) BF_LENGTH(4) BF_LENGTH(5) BF_LENGTH(6) BF_LENGTH(7) BF_LENGTH(8)
+                BF_LENGTH(9) BF_LENGTH(10) BF_LENGTH(11) BF_LENGTH(12) BF_LENGTH(13) BF_LENGTH(14) BF_LENGTH(15)
+                BF_LENGTH(16)
+#undef BF_LENGTH
+                default: {  // one window of 17 to 31 spectra: a lane per beam
+                    float sum = 0.f;
+                    uint32_t at = 0;
+                    int i = 0;
+#pragma unroll 1
+                    for (; i + 8 <= sw; i += 8, at += 512) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) sum += ld_shared_f(row_at[k] + at);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) {
+                        if (i + k < sw) sum += ld_shared_f(row_at[k] + at);
+                    }
+                    if (lane < min(16, beams_left) && wq * sw < jb.n_time) out[lane] = sum;
                 }
             }
         };
@@ -896,6 +921,7 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
             const TcJob& jb = cur.jb;
             const bool short_win = jb.spectra < 32;
             const int sw = jb.spectra, nwin = short_win ? jb.rows_q / sw : 0;
+            if (short_win) set_rows(sw);
             for (int k = un.tile_begin; k < un.tile_end; ++k) {
                 if (!failed && !mbar_wait(&acc_full[acc_stage], acc_phase, kWaitNs)) { fail(128); failed = true; }
                 tc_fence_after();
@@ -921,7 +947,7 @@ grid_tensor_kernel(const __grid_constant__ CUtensorMap vmap, const TcParams p) {
                             if (last) tc_fence_before();
                             __syncwarp();
                             if (last && lane == 0) mbar_arrive(&acc_empty[acc_stage]);
-                            sum_windows(out + 16 * c, jb.n_beams - 16 * (c_begin + c), jb, wq, sw, nwin);
+                            sum_short(out + 16 * c, jb.n_beams - 16 * (c_begin + c), jb, wq, sw);
                             __syncwarp();
                         }
                         released = c_count > 0;

@@ -199,3 +199,16 @@ def test_tensor_grid_128_antennas_every_entry(cuda, orc, A):
     torch.cuda.synchronize()
     assert native.take_device_error() == 0
     assert np.array_equal(integ.cpu().numpy().reshape(got.shape), got)
+
+
+@pytest.mark.parametrize("A,B", [(32, 33), (64, 100)])
+@pytest.mark.parametrize("S", [*range(1, 18), 23, 24, 31])
+def test_every_short_window(cuda, orc, A, B, S):
+    """Each window length below 17 has its own sums, longer ones share a
+    loop: one to three loads per epilogue half, an odd beam count, and a
+    partial last window in the last tile."""
+    T = 270 + S // 2
+    v, w = random_voltage(T, F, A, seed=S), grid_weights(A, F, B, seed=S + 100)
+    from beamform_project_b200 import api
+    got, _, _ = _run(cuda, api, v, w, T, A, B, S, quant=False)
+    _check(orc, got[0], v, w, T, A, B, S)
