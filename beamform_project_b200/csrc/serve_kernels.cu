@@ -6,6 +6,7 @@
 #include "tracker_common.cuh"
 
 #include <climits>
+#include <type_traits>
 
 namespace bf {
 namespace {
@@ -69,15 +70,18 @@ __device__ __forceinline__ int find_job(const long long* begins, int stride_ll, 
 // split at once into the four fp16 parts (re hi, im hi, re lo, im lo) that
 // the fragments hold.  A part row keeps antennas a and a + 2 in one 32-bit
 // word, so each fragment register is one shared-memory load (the im part of
-// a real-row column is the negated word).  Rows are XOR-swizzled so that the
+// a real-row column is the negated word).  Rows are padded so that the
 // 32 lanes of a fragment load hit 32 banks.
 // kShort (windows of at most 16 spectra: one row block) reads the fragments
 // where the MMAs use them instead of holding them in registers, which leaves
 // room for twice the resident CTAs.  Longer windows take the integer form of
-// tracker_common.cuh instead of fp16 parts, an m16n8k32 tile per source, with
-// the eight sources' digit fragments in registers; the plain tracker needs
-// that form, and here it costs what the fp16 form did (a mix of eight jobs,
-// three of them such trackers: 2.67 and 2.63 ms).
+// tracker_common.cuh instead of fp16 parts, two m16n8k32 tiles per pair of
+// sources, with the digit fragments in registers: a lane holds every digit of
+// one component of one source, so putting them together takes no shuffle.
+// Measured through the server, six jobs, eight windows of 320 spectra, 64
+// antennas: 16 sources integrated over 64 spectra 1.16 ms (1.31 with a tile per
+// source, whose lanes put the same digits together twice; 1.15 with fp16
+// parts), over 320 0.84 (0.97; 0.84), one source over 320 0.52 (0.53; 0.58).
 // For one source the arithmetic (weights, fragments, MMA chain, hi + lo
 // combination, window sum order) is that of tracker_stream_kernel, so
 // results agree bit for bit (split(-x) is -split(x) except for the sign of a
@@ -114,13 +118,14 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
     constexpr int kBytes = A / 4;       // bytes (antennas) per thread per spectrum
     using Frag = TrackerFrag<A>;
     constexpr int kWarpWords = 8 * 4 * Frag::kRowWords;  // 8 sources x 4 parts
-    __shared__ double s_delay[2][8][A];  // by unit parity
+    constexpr int kSourceBytes = (kDigitRows + 1) * A;   // the odd row spreads two or four sources over the banks
+    __shared__ __align__(16) double s_delay[2][8][A];  // by unit parity
     // Long windows: the largest |delay| of a source's antennas, and per warp the
     // sources whose weights have no digits (a phase that is not finite, or too
     // large to have a value); their products are NaN.
     __shared__ unsigned s_far[2][8][A / 32], s_no_digits[8];
     // fp16 part rows, or (long windows) the digit rows of four sources at a time
-    __shared__ __align__(16) uint32_t s_frag[8][kShort ? kWarpWords : kDigitRows * A];
+    __shared__ __align__(16) uint32_t s_frag[8][kShort ? kWarpWords : kSourceBytes];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, q = lane & 3;
     const TrJob* jobs = reinterpret_cast<const TrJob*>(table + 1);
@@ -147,7 +152,7 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
     // (source group, then channel group, then window, then job): one job
     // search and two 32-bit divisions per CTA instead of per unit.
     const long long u_begin = n_units * blockIdx.x / gridDim.x;
-    const long long u_end = n_units * (blockIdx.x + 1) / gridDim.x;
+    const int n_mine = static_cast<int>(n_units * (blockIdx.x + 1) / gridDim.x - u_begin);
     int j = 0, sg = 0, fg = 0, w = 0;
     auto seek = [&](long long u) {
         j = find_job(&jobs[0].unit_begin, sizeof(TrJob) / sizeof(long long), n_jobs, u);
@@ -158,14 +163,14 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         fg = static_cast<int>(rest - wq * fgn);
         w = static_cast<int>(wq);
     };
-    if (u_begin < u_end) seek(u_begin);
-    for (long long u = u_begin; u < u_end; ++u) {
-        if (u > u_begin) {
+    if (n_mine > 0) seek(u_begin);
+    for (int i_unit = 0; i_unit < n_mine; ++i_unit) {
+        if (i_unit > 0) {
             if (++sg == jobs[j].src_groups) {
                 sg = 0;
                 if (++fg == jobs[j].fgroups) {
                     fg = 0;
-                    if (++w == jobs[j].n_win) seek(u);  // the next job with units
+                    if (++w == jobs[j].n_win) seek(u_begin + i_unit);  // the next job with units
                 }
             }
         }
@@ -206,7 +211,7 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         // warp writing this unit's buffer has passed the last unit's barrier,
         // which every warp reaches only after forming its weights from this
         // buffer two units ago.
-        const int db = static_cast<int>((u - u_begin) & 1);
+        const int db = i_unit & 1;
         for (int i = threadIdx.x; i < n_here * A; i += blockDim.x) {
             const int sl = i / A, a = i % A;
             const float3 d = trajectory_direction(jb.traj + 4 * (8 * sg + sl), wglob * S);
@@ -254,8 +259,8 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
         }
         __syncwarp();
 
-        // Digit fragments of the long form: column g of source sl's tile.
-        uint32_t bfrag[kShort ? 1 : 8][NW][2];
+        // Digit fragments of the long form: column g of a source pair's two tiles.
+        uint32_t bfrag[kShort ? 1 : 4][2][NW][2];
         if constexpr (!kShort) {
             const double k = fvalid ? jb.kw[f] : 0.0;
             unsigned far = s_far[db][lane & 7][0];
@@ -264,32 +269,43 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
             const unsigned no_digits = ~__ballot_sync(0xffffffffu, phasors);
             if (lane == 0) s_no_digits[warp] = no_digits;
             uint8_t* rows = reinterpret_cast<uint8_t*>(frag);
-            constexpr int kPairs = A / 2, kAtOnce = 32 / kPairs;  // sources formed by a warp at once
+            // kPer antennas per lane: two, or four where that takes 32 antennas'
+            // sources four at a time
+            auto form = [&](auto per, int s0) {
+                constexpr int kPer = decltype(per)::value, kLanes = A / kPer, kAtOnce = 32 / kLanes;
+#pragma unroll 2
+                for (int e = 0; e < 4; e += kAtOnce) {
+                    const int sl = s0 + e + lane / kLanes, at = lane % kLanes;
+                    if (sl < n_here) {
+                        float2 w[kPer];
+#pragma unroll
+                        for (int i = 0; i < kPer; ++i) w[i] = steering_from_delay(k, s_delay[db][sl][kPer * at + i]);
+                        uint8_t* source = rows + (sl - s0) * kSourceBytes;
+                        if constexpr (kPer == 4) store_digit_quad<A>(source, at, w);
+                        else store_digits<A>(source, at, w[0], w[1]);
+                    }
+                }
+            };
 #pragma unroll
             for (int s0 = 0; s0 < 8; s0 += 4) {
                 if (s0 < n_here) {
                     __syncwarp();  // the last four sources' rows are read
-#pragma unroll 1
-                    for (int e = 0; e < 4; e += kAtOnce) {
-                        const int sl = s0 + e + lane / kPairs, pair = lane % kPairs;
-                        if (sl < n_here) {
-                            store_digits<A>(rows + (sl - s0) * kDigitRows * A, pair,
-                                            steering_from_delay(k, s_delay[db][sl][2 * pair]),
-                                            steering_from_delay(k, s_delay[db][sl][2 * pair + 1]));
-                        }
-                    }
+                    if (A == 32 && n_here - s0 > 2) form(std::integral_constant<int, 4>{}, s0);
+                    else form(std::integral_constant<int, 2>{}, s0);
                     __syncwarp();
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (s0 + e < n_here) load_digit_frags<A>(rows + e * kDigitRows * A, g, q, bfrag[s0 + e]);
+                    for (int e = 0; e < 4; e += 2) {
+                        if (s0 + e < n_here) {
+                            const uint8_t* first = rows + e * kSourceBytes;
+                            load_pair_frags<A>(first, s0 + e + 1 < n_here ? first + kSourceBytes : first, g, q,
+                                               bfrag[(s0 + e) / 2]);
+                        }
                     }
                 }
             }
         }
 
-        float pw[kShort ? 4 : 8];
-#pragma unroll
-        for (int i = 0; i < (kShort ? 4 : 8); ++i) pw[i] = 0.f;
+        float pw[4] = {0.f, 0.f, 0.f, 0.f};
         for (int tb = t_begin; tb < t_end; tb += 16) {
             uint32_t ng[NW], ng8[NW];
             if constexpr (!kShort) load_rows(tb + 16, ng, ng8);
@@ -337,16 +353,24 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
                     im[1][jj] = word_im16(wg8[jj]);
                 }
 #pragma unroll
-                for (int sl = 0; sl < 8; ++sl) {
-                    if (sl < n_here) {
-                        int d[4] = {0, 0, 0, 0};
+                for (int nt = 0; nt < 4; ++nt) {
+                    if (nt < n_tiles) {
+                        int hi[4] = {0, 0, 0, 0}, lo[4] = {0, 0, 0, 0};
 #pragma unroll
                         for (int jj = 0; jj < NW; ++jj) {
-                            mma_16832(d, re[0][jj], re[1][jj], im[0][jj], im[1][jj], bfrag[sl][jj][0], bfrag[sl][jj][1]);
+                            mma_16832(hi, re[0][jj], re[1][jj], im[0][jj], im[1][jj], bfrag[nt][0][jj][0],
+                                      bfrag[nt][0][jj][1]);
+                            mma_16832(lo, re[0][jj], re[1][jj], im[0][jj], im[1][jj], bfrag[nt][1][jj][0],
+                                      bfrag[nt][1][jj][1]);
                         }
-                        float sq_g, sq_h;
-                        digit_squares<A>(d, digit_scale(q), sq_g, sq_h);
-                        pw[sl] = __fadd_rn(pw[sl], __fadd_rn(sq_g, sq_h));  // re^2 and im^2 apart until the window ends
+                        // 2^18 x the component of rows g and g + 8: the rounding of
+                        // digit_squares, its scale left to the end of the window
+                        const float f_g = __fmaf_rn(__int2float_rn(lo[0] * 256 + lo[1]), 0x1p-16f,
+                                                    __int2float_rn(hi[0] * 256 + hi[1]));
+                        const float f_h = __fmaf_rn(__int2float_rn(lo[2] * 256 + lo[3]), 0x1p-16f,
+                                                    __int2float_rn(hi[2] * 256 + hi[3]));
+                        // re^2 and im^2 apart until the window ends
+                        pw[nt] = __fadd_rn(pw[nt], __fadd_rn(__fmul_rn(f_g, f_g), __fmul_rn(f_h, f_h)));
                     }
                 }
             }
@@ -359,16 +383,17 @@ served_tracker_kernel(const uint8_t* __restrict__ pool, long long row_stride, co
             }
         }
 #pragma unroll
-        for (int i = 0; i < (kShort ? 4 : 8); ++i) {
-            if (i < (kShort ? n_tiles : n_here)) {
-                float acc = pw[i];
+        for (int nt = 0; nt < 4; ++nt) {
+            if (nt < n_tiles) {
+                float acc = pw[nt];
                 if constexpr (!kShort) acc += __shfl_xor_sync(0xffffffffu, acc, 2);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 4);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 8);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 16);
-                if (!kShort && ((s_no_digits[warp] >> i) & 1u) != 0) acc = NAN;
-                const int src = 8 * sg + (kShort ? 2 * i + (q >> 1) : i);
-                if (g == 0 && (kShort ? (q & 1) == 0 : q == 0) && fvalid && src < n_src) {
+                // the tile's sources: in lanes 0 and 2, long windows in lanes 0 and 1
+                const int sl = 2 * nt + (kShort ? q >> 1 : q & 1), src = 8 * sg + sl;
+                if constexpr (!kShort) acc = ((s_no_digits[warp] >> sl) & 1u) != 0 ? NAN : acc * 0x1p-36f;
+                if (g == 0 && (kShort ? (q & 1) == 0 : q < 2) && fvalid && src < n_src) {
                     jb.integrated[(wglob * jb.n_freq + f) * n_src + src] = acc;
                 }
             }

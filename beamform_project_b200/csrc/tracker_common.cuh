@@ -169,12 +169,34 @@ __device__ __forceinline__ void store_digits(uint8_t* rows, int pair, float2 w0,
         dst[(8 + d) * (A / 2)] = static_cast<uint16_t>(__byte_perm(y0.pos, y1.pos, sel));
     }
 }
-// B fragments (b0: re inputs, b1: im inputs) of column g of the MMAs over word
-// j of every lane quad's A / 4 antennas.
+// Antennas 4 quad .. + 3 of the rows.
 template <int A>
-__device__ __forceinline__ void load_digit_frags(const uint8_t* rows, int g, int q, uint32_t (&b)[A / 16][2]) {
-    const uint8_t* r0 = rows + (g < 4 ? g : g + 4) * A + q * (A / 4);  // re: Re w; im: Im w
-    const uint8_t* r1 = rows + (g < 4 ? g + 4 : g - 4) * A + q * (A / 4);  // re: -Im w; im: Re w
+__device__ __forceinline__ void store_digit_quad(uint8_t* rows, int quad, const float2 (&w)[4]) {
+    uint32_t words[3][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const Digits im = weight_digits(w[a].y);
+        words[0][a] = weight_digits(w[a].x).pos;
+        words[1][a] = im.neg;
+        words[2][a] = im.pos;
+    }
+    uint32_t* dst = reinterpret_cast<uint32_t*>(rows) + quad;
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+        // bytes 0 and 1, 2 and 3 of two antennas, then each byte of all four
+        const uint32_t* x = words[part];
+        const uint32_t lo0 = __byte_perm(x[0], x[1], 0x5140), lo1 = __byte_perm(x[2], x[3], 0x5140);
+        const uint32_t hi0 = __byte_perm(x[0], x[1], 0x7362), hi1 = __byte_perm(x[2], x[3], 0x7362);
+        dst[(4 * part) * (A / 4)] = __byte_perm(hi0, hi1, 0x7632);
+        dst[(4 * part + 1) * (A / 4)] = __byte_perm(hi0, hi1, 0x5410);
+        dst[(4 * part + 2) * (A / 4)] = __byte_perm(lo0, lo1, 0x7632);
+        dst[(4 * part + 3) * (A / 4)] = __byte_perm(lo0, lo1, 0x5410);
+    }
+}
+// B fragments (b0: re inputs, b1: im inputs) of a column's two rows, over word
+// j of the A / 4 antennas of a lane quad.
+template <int A>
+__device__ __forceinline__ void load_row_frags(const uint8_t* r0, const uint8_t* r1, uint32_t (&b)[A / 16][2]) {
     if constexpr (A == 32) {
         const uint2 x = *reinterpret_cast<const uint2*>(r0), y = *reinterpret_cast<const uint2*>(r1);
         b[0][0] = x.x; b[1][0] = x.y; b[0][1] = y.x; b[1][1] = y.y;
@@ -185,6 +207,25 @@ __device__ __forceinline__ void load_digit_frags(const uint8_t* rows, int g, int
             b[j][0] = x.x; b[j + 1][0] = x.y; b[j + 2][0] = x.z; b[j + 3][0] = x.w;
             b[j][1] = y.x; b[j + 1][1] = y.y; b[j + 2][1] = y.z; b[j + 3][1] = y.w;
         }
+    }
+}
+// One source: column g of (re, im) x (d3, d2, d1, d0).
+template <int A>
+__device__ __forceinline__ void load_digit_frags(const uint8_t* rows, int g, int q, uint32_t (&b)[A / 16][2]) {
+    load_row_frags<A>(rows + (g < 4 ? g : g + 4) * A + q * (A / 4),       // re: Re w; im: Im w
+                      rows + (g < 4 ? g + 4 : g - 4) * A + q * (A / 4), b);  // re: -Im w; im: Re w
+}
+// Two sources: columns (re, im) x (first, second source) x two digits, d3 and
+// d2 in one tile, d1 and d0 in the other, so that a lane holds all digits of
+// one component of one source.
+template <int A>
+__device__ __forceinline__ void load_pair_frags(const uint8_t* first, const uint8_t* second, int g, int q,
+                                                uint32_t (&b)[2][A / 16][2]) {
+    const uint8_t* rows = ((g & 2) == 0 ? first : second) + q * (A / 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int d = 2 * h + (g & 1);
+        load_row_frags<A>(rows + (g < 4 ? d : d + 8) * A, rows + (g < 4 ? d + 4 : d) * A, b[h]);
     }
 }
 __device__ __forceinline__ void mma_16832(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,

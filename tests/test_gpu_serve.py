@@ -320,3 +320,12 @@ def test_served_tracker_without_a_phase(cuda, A, S):
     nan = np.isnan(b).reshape(-1, 11)
     assert not nan[:, zenith].any() and np.delete(nan, zenith, axis=1).all()
     assert np.array_equal(b.reshape(-1, 11)[:, zenith], a.reshape(-1, 11)[:, zenith])
+
+
+@pytest.mark.parametrize("A", [32, 64])
+@pytest.mark.parametrize("n_src,S", [(1, 20), (2, 32), (3, 64), (4, 20), (5, 160), (7, 32), (8, 320), (9, 40), (12, 20)])
+def test_served_sources_in_pairs(cuda, A, n_src, S):
+    """Long windows take sources in pairs, formed two or four at a time and
+    eight to a unit: whole pairs and odd ones out, on both sides of four and
+    of eight."""
+    test_served_tracker_equals_plain_tracker(cuda, A, S, n_src)
