@@ -12,10 +12,13 @@
 // (channel, group of up to 64 beams, run of whole windows) and walks the run
 // in tiles of 64 spectra.  A warp owns 8 spectra of the tile and every beam
 // of the group: lane = (one of 8 beam columns, one of 4 spectrum pairs), with
-// BL beams per lane.  Two beams at a time share packed f32x2 registers, so a
-// complex multiply-add of two beams is eight packed instructions, each
-// rounding its halves as the scalar instruction would; the last beam of an
-// odd BL packs the pair's two spectra instead.  Weights sit in shared memory
+// BL beams per lane.  (Short blocks take CTAs of 2 warps and tiles of 16
+// spectra, where a warp without spectra does no arithmetic: one spectrum of
+// 128 beams at 64 antennas 26.6 us, 65.5 with the tile of 64.)  Two beams at a
+// time share packed f32x2 registers, so a complex multiply-add of two beams is
+// eight packed instructions, each rounding its halves as the scalar
+// instruction would; the last beam of an odd BL packs the pair's two spectra
+// instead.  Weights sit in shared memory
 // as (re, re, im, im) of two beams and voltages as (re, re, im, im) of two
 // spectra per antenna: BL / 2 + 1 loads of 16 bytes per lane feed 8 BL packed
 // instructions.  The weights stay for the CTA's life (32 beams a group at 256
@@ -42,11 +45,17 @@
 namespace bf {
 namespace {
 
-constexpr int kWarps = 8;
-constexpr int kThreads = 32 * kWarps;
-constexpr int kTile = 8 * kWarps;     // spectra per tile: four pairs per warp
-constexpr int kPairs = kTile / 2;
+constexpr int kWarps = 8;             // warps of a CTA, and of one for a short block
+constexpr int kShortWarps = 2;
+constexpr int tile_spectra(int warps) { return 8 * warps; }  // four pairs per warp
+constexpr int kTile = tile_spectra(kWarps);
 constexpr int kChunk = 64;            // antennas staged at once
+// Longest block of the short form: its CTAs are a quarter of the size, so more
+// of them hide one another's latency while most of a 64-spectrum tile would be
+// empty.  64 beams, 64 antennas: 16 spectra 16.4 us (30.7 in the long form), 32
+// 24.6 (32.2); 128 antennas 16 28.7 (49.2), but 32 of 128 beams 93.9 (86.1: two
+// tiles per CTA, and the weights leave room for five on an SM).
+__host__ __device__ constexpr int short_block(uint64_t n_ant) { return n_ant <= 64 ? 32 : 16; }
 // Beams per CTA: up to 64, with the weights of every antenna in half an SM's
 // shared memory.
 __host__ __device__ constexpr int max_group(uint64_t n_ant) { return n_ant <= 128 ? 64 : 32; }
@@ -64,8 +73,9 @@ struct ExactParams {
     float one;              // 1
 };
 
-template <int BL>
-__global__ void __launch_bounds__(kThreads, 2) grid_exact_kernel(const ExactParams p) {
+template <int BL, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS) grid_exact_kernel(const ExactParams p) {
+    constexpr int kThreads = 32 * WARPS, kTile = tile_spectra(WARPS), kPairs = kTile / 2;
     constexpr int kBeams = 8 * BL;
     constexpr int JP = BL / 2;             // beam pairs per lane: beams 16 j + 2 col and the next
     constexpr bool kOdd = (BL & 1) != 0;   // and beam 16 JP + col
@@ -211,6 +221,9 @@ __global__ void __launch_bounds__(kThreads, 2) grid_exact_kernel(const ExactPara
         }
         // the warp's four pairs read antenna a from four different bank groups
         const float4* xrow = xs + pair * AC;
+        // a warp without spectra in the tile (in the long form the test costs more
+        // than it saves: 1 % of long blocks)
+        if (WARPS == kShortWarps && t_begin + step / chunks * kTile + 8 * warp >= t_end) continue;
 #pragma unroll 1
         for (int a0 = 0; a0 < AC; a0 += 8) {
 #pragma unroll
@@ -258,20 +271,26 @@ __global__ void __launch_bounds__(kThreads, 2) grid_exact_kernel(const ExactPara
     if (p.spectra > 0 && lb < kBeams && left < p.spectra) finish_window();  // partial last window
 }
 
+template <int BL, int WARPS>
+bf_status launch_exact(cudaStream_t stream, const ExactParams& p, unsigned blocks) {
+    const int AC = p.n_ant < kChunk ? p.n_ant : kChunk;
+    const int smem = (p.n_ant * 4 * BL + tile_spectra(WARPS) / 2 * AC) * static_cast<int>(sizeof(float4)) +
+                     tile_spectra(WARPS) * (8 * BL + 4) * static_cast<int>(sizeof(float));
+    cudaError_t err =
+        cudaFuncSetAttribute(grid_exact_kernel<BL, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return cuda_status(err, "grid_exact_kernel smem attribute");
+    grid_exact_kernel<BL, WARPS><<<blocks, 32 * WARPS, smem, stream>>>(p);
+    return cuda_status(cudaGetLastError(), "grid_exact_kernel launch");
+}
+
 template <int BL>
 bf_status launch_beams(int bl, cudaStream_t stream, const ExactParams& p, unsigned blocks) {
     if constexpr (BL > 8) {
         return set_error(BF_ERR_LOGIC, "beam group out of range");
     } else {
         if (bl != BL) return launch_beams<BL + 1>(bl, stream, p, blocks);
-        const int AC = p.n_ant < kChunk ? p.n_ant : kChunk;
-        const int smem = (p.n_ant * 4 * BL + kPairs * AC) * static_cast<int>(sizeof(float4)) +
-                         kTile * (8 * BL + 4) * static_cast<int>(sizeof(float));
-        cudaError_t err =
-            cudaFuncSetAttribute(grid_exact_kernel<BL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (err != cudaSuccess) return cuda_status(err, "grid_exact_kernel smem attribute");
-        grid_exact_kernel<BL><<<blocks, kThreads, smem, stream>>>(p);
-        return cuda_status(cudaGetLastError(), "grid_exact_kernel launch");
+        return p.n_time <= short_block(p.n_ant) ? launch_exact<BL, kShortWarps>(stream, p, blocks)
+                                                : launch_exact<BL, kWarps>(stream, p, blocks);
     }
 }
 

@@ -165,3 +165,13 @@ def test_tile_edges_bit_exact(cuda, orc, A, B, T, S, kernel):
         api.launch_packed_beamformer(kernel, None, dv, dw, out, d)
         exp = orc.beamform(v, w, T, F, A, B)
     assert np.array_equal(out.cpu().numpy().reshape(W, F, B), exp)
+
+
+@pytest.mark.parametrize("A,B,T,S", [(64, 128, 1, 0), (64, 64, 8, 0), (32, 9, 9, 7), (64, 65, 15, 15), (128, 33, 16, 10),
+                                     (256, 128, 16, 0), (256, 1, 1, 1), (128, 40, 17, 0), (32, 128, 31, 10),
+                                     (64, 8, 32, 32), (64, 63, 33, 0), (32, 37, 26, 3)])
+@pytest.mark.parametrize("kernel", [0, 1])
+def test_short_blocks_bit_exact(cuda, orc, A, B, T, S, kernel):
+    """Blocks around the spectra of a warp (8), of the short form's tile (16)
+    and of its longest block (16, 32 up to 64 antennas)."""
+    test_tile_edges_bit_exact(cuda, orc, A, B, T, S, kernel)
