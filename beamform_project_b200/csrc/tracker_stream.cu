@@ -412,8 +412,11 @@ bf_status launch_stream(cudaStream_t stream, const uint8_t* v, const float* pos,
     auto kernel = !runs  ? tracker_stream_kernel<A, false, true>
                   : int8 ? tracker_stream_kernel<A, true, true>
                          : tracker_stream_kernel<A, true, false>;
-    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    if (err != cudaSuccess) return cuda_status(err, "tracker_stream_kernel smem attribute");
+    if (smem > 48 * 1024) {  // the limit of a launch that asks for no more; asking costs 0.5 us
+        cudaError_t err =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (err != cudaSuccess) return cuda_status(err, "tracker_stream_kernel smem attribute");
+    }
     const dim3 grid(static_cast<unsigned>((W + run - 1) / run), static_cast<unsigned>(channel_groups));
     kernel<<<grid, kChannelsPerCta * 32, smem, stream>>>(v, pos, k, dirs, intensity, integrated, T, F, S, W, run);
     return cuda_status(cudaGetLastError(), "tracker_stream_kernel launch");
