@@ -26,6 +26,9 @@ inline bf_status cuda_status(cudaError_t err, const char* what) {
     return set_error(BF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(err));
 }
 
+// Channels of a shard, the count every entry but the channel slices takes.
+constexpr uint64_t kShardChannels = 336;
+
 // validate_dimensions (include/beamformer/config.hpp:81-94).
 bf_status validate_dims(const bf_dims* dims);
 

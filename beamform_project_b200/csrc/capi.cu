@@ -33,7 +33,7 @@ bf_status clear_error() {
 bf_status validate_dims(const bf_dims* dims) {
     if (dims == nullptr) return set_error(BF_ERR_INVALID_ARGUMENT, "dims must not be null");
     if (dims->n_time == 0) return set_error(BF_ERR_INVALID_ARGUMENT, "n_time must be positive");
-    if (dims->n_freq != 336) {
+    if (dims->n_freq != kShardChannels) {
         return set_error(BF_ERR_INVALID_ARGUMENT,
                          "the local-shard contract requires exactly 336 frequency channels");
     }

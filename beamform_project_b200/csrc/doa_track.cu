@@ -111,6 +111,7 @@ constexpr int kCoarseTile = 16;      // coarse points per cluster
 constexpr int kFine = 9;             // candidates of a refinement
 constexpr int kSearchThreads = kFine * kChanGroup;
 constexpr int kMaxGroups = 8;        // CTAs per cluster (a portable cluster)
+static_assert(kShardChannels <= kMaxGroups * kChanGroup, "a shard's channels fit one cluster");
 
 struct SearchParams {
     int levels, G;
@@ -417,7 +418,6 @@ bf_status launch_doa_track(cudaStream_t stream, const uint8_t* v, const float* p
     const int M = static_cast<int>((c.subarray > 0 && c.subarray < A) ? c.subarray : A);
     if (M > kMaxM) return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 16 elements after smoothing");
     const uint64_t groups = (F + kChanGroup - 1) / kChanGroup;
-    if (groups > kMaxGroups) return set_error(BF_ERR_UNSUPPORTED, "the DOA search supports at most 512 channels");
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     auto* R = reinterpret_cast<int32_t*>(ws);
     ws += align256(static_cast<uint64_t>(B) * F * A * A * 2 * sizeof(int32_t));
