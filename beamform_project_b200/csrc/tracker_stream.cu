@@ -63,7 +63,12 @@ using namespace trk;
 
 constexpr int kChannelsPerCta = 8;
 constexpr int kMaxRun = 16;         // windows per CTA
-constexpr int kRunSpectra = 160;    // a run is as many windows as fit, one at least
+// A run is as many windows as fit in these spectra, one at least: enough for two
+// windows of the longest length, whose weights and first loads then overlap the
+// window before (with 80, windows of 64 were 3 to 8 % slower, of 16 3 %; with
+// 320 none was faster).  Half of kMaxRun made windows of 1 3 % slower at 64
+// antennas.
+constexpr int kRunSpectra = 160;
 constexpr int kWantedCtas = 4 * 4 * 148;
 // Longest window of the ring form: in the fp16 form windows of 100 took 75 us
 // in it and 77 us in the long form (9999 spectra), windows of 320 179 and 166
