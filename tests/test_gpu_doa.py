@@ -269,6 +269,8 @@ def test_adaptive_tracker_follows_reference_search(cuda, ref, orc, A, capon, sub
         assert np.array_equal(got_I[w * K:(w + 1) * K], ref_I[w * K:(w + 1) * K])
 
 
+# The search kernel's point tile is 16 per cluster, and the powers of every cell
+# are in the workspace: 9 x 9 leaves a tile of one point, 24 x 24 full tiles.
 @pytest.mark.gpu
 @pytest.mark.parametrize("G,M,capon", [(9, 8, False), (24, 12, False), (24, 5, True), (3, 16, True)])
 def test_adaptive_tracker_takes_the_grid_maximum(cuda, orc, G, M, capon):

@@ -7,6 +7,8 @@ kernel, fp16 hi+lo weights, fp32 sums) must match within the reference's
 CUDA tolerance |gpu - cpu| <= 1e-3 + 1e-5 |cpu| (tests/cuda/
 test_cuda_packed.cu:24-25), and its per-window sums within 1e-5 relative of
 the FP64 sum.
+The fp16 weights are those of windows of up to 16 spectra; longer windows take
+int8 digits of the weights and are held to the same bars.
 """
 from __future__ import annotations
 
