@@ -23,6 +23,8 @@
 #include "bf_internal.cuh"
 #include "packed_f32.cuh"
 
+#include <algorithm>
+
 namespace bf {
 
 bf_status launch_tracker_stream(cudaStream_t stream, const uint8_t* v, const float* pos,
@@ -131,7 +133,8 @@ bf_status launch_tracker(cudaStream_t stream, int mode, const uint8_t* v, const 
     const dim3 grid(static_cast<unsigned>(W), static_cast<unsigned>((d.n_freq + 31) / 32));
     tracker_exact_kernel<<<grid, kSlots * 32, smem, stream>>>(
         v, pos, k, dirs, intensity, integrated, static_cast<int>(d.n_time),
-        static_cast<int>(d.n_freq), static_cast<int>(d.n_ant), static_cast<int>(spectra), 1.0f);
+        static_cast<int>(d.n_freq), static_cast<int>(d.n_ant),
+        static_cast<int>(std::min<uint64_t>(spectra, d.n_time)), 1.0f);
     return cuda_status(cudaGetLastError(), "tracker_exact_kernel launch");
 }
 

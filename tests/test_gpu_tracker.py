@@ -150,3 +150,16 @@ def test_mode1_not_finite(cuda, orc, A, S):
     for g, b, o, e in zip(good, bad, order, expect):
         assert np.array_equal(np.isnan(b), e) and np.array_equal(np.isnan(o), e)
         assert np.array_equal(b[~e], g[~e])
+
+
+@pytest.mark.parametrize("S", [2**31, 2**32, 2**32 + 5])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_window_longer_than_32_bits(cuda, orc, mode, S):
+    """An integration length past 32 bits is one window, as any length past
+    the run is."""
+    from beamform_project_b200 import api
+    A, T = 64, 50
+    pos, freq, dirs, v, _ = _case(orc, api, T, A, T, seed=3)
+    whole, longer = (_run(cuda, api, mode, v, pos, freq, dirs, T, A, s) for s in (T, S))
+    for a, b in zip(whole, longer):
+        assert np.array_equal(a, b)
